@@ -46,11 +46,11 @@ int rgs_debug_forward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_
 int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera* camera, const float* target_rgba,
                        const float bg[3], float lambda, float* acc9, float* dl_dpix);
 
-/* Largest relative difference between the backward blend's SFU exponential
- * and the forward's exact exp (the one the oracle restates) over n points on
- * [lo, hi], -8 <= lo <= hi <= 0: the bound behind the backward's rule of
- * deciding alpha >= 1/255 and alpha > 0.99 with the exact exp whenever the
- * SFU value lies within 4e-6 relative of either threshold. */
+/* Largest relative difference between the SFU exponential the backward blend
+ * forms its alphas with and the forward's exact exp (the one the oracle
+ * restates) over n points on [lo, hi], -8 <= lo <= hi <= 0. (Which splats
+ * contribute is decided on the exponent, with the forward's own arithmetic
+ * wherever the two evaluations could disagree.) */
 int rgs_debug_exp_sfu_error(rgs_ctx* ctx, float lo, float hi, uint32_t n, float* max_rel);
 
 /* Pixels of the view at position k of the trainer's most recent batched pass

@@ -29,10 +29,9 @@
 //     about five instructions per pixel, less than the strip tests add to
 //     every staging round.)
 //   * backward warps skip splats past the warp's largest last_contrib.
-// Backward pre-reduces each splat's 9 partial gradients across the warp with
-// shuffles (only when a lane contributed), across warps with shared-memory
-// atomics, and issues one 3 x 16-byte vector reduction (red.global.add.v4.f32)
-// per splat per CTA.
+// Backward gathers each warp's partial gradients of eight splats in shared
+// memory, reads them back transposed (four lanes per splat) and issues one
+// 3 x 16-byte vector reduction (red.global.add.v4.f32) per splat per warp.
 //
 // CTA tiles other than 16x16 keep the reference's per-pixel semantics: each
 // record carries its reference-tile rectangle in pixels and a pixel only
@@ -62,10 +61,10 @@ __device__ __forceinline__ bool in_rect(float rx, float ry, int px, int py) {
 // li0 is the tile-list index of `first`. Must be called by the whole block.
 // When s_rall is given, every staged entry's pixel rectangle (kept or not) is
 // recorded at its batch position.
-template <int NT, int BATCH, int RW, bool WMASK>
+template <int NT, int BATCH>
 __device__ __forceinline__ int stage_batch(const BlendArgs& a, size_t S, uint32_t first, uint32_t end, int li0, float x0c,
-                                           float x1c, float y0c, float y1c, int ytile, int height, float4* s_a, float4* s_c,
-                                           float4* s_k, int* s_li, uint8_t* s_wm, uint32_t* s_slot, int* s_wsum, uint2* s_rall) {
+                                           float x1c, float y0c, float y1c, float4* s_a, float4* s_c, float4* s_k, int* s_li,
+                                           int* s_wsum, uint2* s_rall) {
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     int kept = 0;
@@ -75,27 +74,14 @@ __device__ __forceinline__ int stage_batch(const BlendArgs& a, size_t S, uint32_
         const uint32_t idx = first + (uint32_t)j;
         bool keep = false;
         float4 A, Q, K;
-        uint32_t slot = 0, wm = 0;
         if (j < BATCH && idx < end) {
-            slot = a.pair_vals[idx];
+            const uint32_t slot = a.pair_vals[idx];
             A = a.rec[slot];
             Q = a.rec[S + slot];
             K = a.rec[2 * S + slot];
             A.w = power_floor(A.z);
             const TileTest t = tile_test_setup(A.x, A.y, Q.x, Q.y, Q.z, A.w);
             keep = !tile_rejects(t, x0c, x1c, y0c, y1c);
-            if (WMASK && keep) {
-                // warp ww owns pixel rows [ww*RW, ww*RW + RW) of the tile: keep the
-                // warps the tile test cannot reject on their own strip of pixel
-                // centres (strips past the image hold no pixel)
-#pragma unroll
-                for (int ww = 0; ww < NW; ++ww) {
-                    const int r0 = ytile + ww * RW;
-                    if (r0 >= height) continue;
-                    const float sy0 = (float)r0 + 0.5f, sy1 = (float)(min(r0 + RW, height) - 1) + 0.5f;
-                    if (!tile_rejects(t, x0c, x1c, sy0, sy1)) wm |= 1u << ww;
-                }
-            }
             if (s_rall) s_rall[j] = make_uint2(__float_as_uint(Q.w), __float_as_uint(K.w));
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -114,8 +100,6 @@ __device__ __forceinline__ int stage_batch(const BlendArgs& a, size_t S, uint32_
             s_c[p] = Q;
             s_k[p] = K;
             s_li[p] = li0 + j;
-            if (WMASK) s_wm[p] = (uint8_t)wm;
-            if (s_slot) s_slot[p] = slot;
         }
         kept += total;
         __syncthreads();
@@ -150,7 +134,6 @@ __global__ void __launch_bounds__(TW * TH / PPT) k_blend_fwd(BlendArgs a) {
     __shared__ uint2 s_rall[RECT ? BATCH : 1];
     __shared__ __align__(16) float2 s_row[ROWTERMS ? BATCH : 1][ROWTERMS ? TH : 1];  // (dy, Q.z*dy*dy)
     __shared__ int s_tile;
-    constexpr int RW = (32 / TW) * PPT;  // pixel rows per warp
     const int tid = threadIdx.x;
     const int total_tiles = a.total_tiles ? (int)*a.total_tiles : a.total_tiles_host;
     const size_t S = (size_t)a.n_per_view * a.nviews;
@@ -189,9 +172,8 @@ __global__ void __launch_bounds__(TW * TH / PPT) k_blend_fwd(BlendArgs a) {
         for (uint32_t b0 = rg.x; b0 < rg.y; b0 += BATCH) {
             if (__syncthreads_count(!all_done) == 0) break;
             const bool need_seen = RECT && a.empty_tile_black;
-            const int nb = stage_batch<NT, BATCH, RW, false>(a, S, b0, rg.y, (int)(b0 - rg.x), x0c, x1c, y0c, y1c, ty * TH,
-                                                             c.height, s_a, s_c, s_k, s_li, nullptr, nullptr, s_wsum,
-                                                             need_seen ? s_rall : nullptr);
+            const int nb = stage_batch<NT, BATCH>(a, S, b0, rg.y, (int)(b0 - rg.x), x0c, x1c, y0c, y1c, s_a, s_c, s_k, s_li,
+                                                  s_wsum, need_seen ? s_rall : nullptr);
             if (need_seen) {
                 // a pixel's reference tile list is non-empty iff some entry (kept
                 // or rejected) covers the pixel
@@ -324,79 +306,92 @@ __global__ void __launch_bounds__(TW * TH / PPT) k_blend_fwd(BlendArgs a) {
 }
 
 
-// Warp sum of nine per-lane values, added into dst[0..8] in shared memory.
-// Values 0..7 are reduced with a transpose (reduce-scatter) pattern: at each
-// xor step a lane keeps half of its values and trades the other half, so after
-// three steps lane l holds value l >> 2 summed over the lanes that differ in
-// bits 4..2, and two more steps finish it: 14 shuffles in place of 45, and
-// eight lanes then add distinct addresses in one instruction.
-__device__ __forceinline__ void warp_reduce_scatter9(const float (&g)[9], int lane, float* dst) {
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-    float w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float send = b4 ? g[i] : g[i + 4];
-        const float keep = b4 ? g[i + 4] : g[i];
-        w[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-    float x[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float send = b3 ? w[i] : w[i + 2];
-        const float keep = b3 ? w[i + 2] : w[i];
-        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    float y = (b2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, b2 ? x[0] : x[1], 4);
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    float z = g[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    if ((lane & 3) == 0) atomicAdd(dst + (lane >> 2), y);
-    if (lane == 0) atomicAdd(dst + 8, z);
-}
-
 __device__ __forceinline__ void red_add_v4(float4* addr, float x, float y, float z, float w) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
+// One pixel of the backward decided with the forward's own arithmetic: nal is
+// minus its alpha (0 when it does not take the splat) and um minus the raw
+// alpha that scales dL/dalpha (0 when the raw alpha was clamped,
+// backward.rs:459-461). A NaN power passes both tests and fminf turns it into
+// alpha = 0.99, as in the forward. Kept out of line: a few pixels in 10^5 come
+// here.
+__device__ __noinline__ float2 bwd_exact_pixel(float dx, float dy, float4 q, float thr) {
+    const float tdx = q.x * dx * dx;
+    const float t2b = 2.0f * q.y * dx;
+    const float power = -0.5f * (tdx + t2b * dy + q.z * dy * dy);
+    if (power > 0.0f || power < thr) return make_float2(0.0f, 0.0f);
+    const float ar = q.w * expf_fast_nonpos(power);
+    const float al = fminf(ar, 0.99f);
+    if (al < 1.0f / 255.0f) return make_float2(0.0f, 0.0f);
+    return make_float2(-al, ar > 0.99f ? 0.0f : -ar);
+}
 
-// Backward. A thread owns PPT vertical pixels; their gradient contributions to
-// a splat are summed in registers before the warp reduction. T is rebuilt as
-// T * 1/(1 - alpha) with the hardware reciprocal (within 2 ulp; one reciprocal
-// serves both uses, where the reference divides, backward.rs:452): over the
-// at most few hundred splats a pixel rebuilds through, T stays within ~1e-5
-// relative of the reference's, far inside the gradients' 1e-3 tolerance.
-// Alpha is formed with the SFU exponential (within 1e-6 of the forward's
-// value); wherever that value lies within 4e-6 relative of the 1/255 cut or
-// the 0.99 clamp, the forward's exact exp decides instead, so the set of
-// contributing splats and the clamped ones are exactly the forward's.
-// The register budget is capped for occupancy: eight 128-thread CTAs per SM
-// with two pixels per thread, twelve 64-thread CTAs with four (a few spilled
-// words cost less than the lost warps: measured 2 % and 10 % faster backward
-// passes on the 1M-Gaussian step; fourteen or sixteen 64-thread CTAs, at 72
-// or 64 registers with more spilling, took 3.39 and 4.31 ms against 3.22).
-template <int TW, int TH, int BATCH, bool RECT, int PPT, bool STORE = false>
-__global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 8 : PPT == 4 ? 12 : 1) k_blend_bwd(BlendArgs a) {
+// Backward. A thread owns PPT vertical pixels in packed f32x2 lanes; T is
+// rebuilt as T * 1/(1 - alpha) with the hardware reciprocal (within 2 ulp; the
+// reference divides, backward.rs:452).
+//
+// What bounds it: instruction issue (70 % of cycles; FMA pipe 42 %, ALU 37 %),
+// so the loop is built around the fewest instructions per (warp, splat). It
+// replaces a loop that tested both thresholds on each pixel's alpha and reduced
+// nine sums over the warp for every splat: 3.29 -> 1.60 ms on 1M Gaussians x 8
+// views, 1.57 -> 0.60 ms on 97k x 3 views of 1277x719 with a white background,
+// 262 -> 70 us on 10k at 256x256 (where one tile's serial walk is the time).
+//
+// Alpha comes from one SFU exponential of p = power log2(e) + log2(opacity),
+// with the power rounded exactly as the forward rounds it. (A power from two
+// packed FMAs over prescaled coefficients saves four packed instructions per
+// pixel pair and ran 4 % faster; but an ill-conditioned conic's terms cancel,
+// and its alpha then strays from the forward's by up to 1e-4.) The
+// contributing set must be the forward's exactly, so a pixel whose p lies
+// within BWD_BAND of a decision (alpha >= 1/255; alpha_raw > 0.99; power > 0,
+// where p reaches log2(opacity)) is decided by bwd_exact_pixel: the roundings
+// of p (|p| <= 8), of log2(opacity) and of the forward's own alpha add up to
+// less than 2e-6 in log2 units, half the band. Every test reads a NaN as
+// "decide exactly".
+//
+// The nine gradient sums of a splat are not reduced across the warp per splat
+// (14 shuffles and two shared atomics each, serialised): a lane stores its six
+// column sums (colour x3, u, u dy, u dy^2 with u = dL/dpower) for up to
+// BWD_GRP splats in the warp's own shared memory, then the warp reads them
+// transposed, four lanes per splat, each adding eight columns, expands the
+// moments in dx, and issues one red.global.add.v4 per accumulator plane. The
+// stores and loads are swizzled by the splat's place in the group, so neither
+// has bank conflicts. Warps share only the staged batch and the two barriers
+// around it.
+//
+// Every lane of a warp that some lane's pixels need runs the whole update (its
+// terms are zero); a branch per thread ran 4 % slower. Ten CTAs per SM (96
+// registers) with four pixels per thread: 11 and 12 ran 3 % and 5 % slower.
+// 64 staged splats: 128 ran 3 % slower. Also measured slower: coefficients
+// stored twice so that a 16-byte load fills both lanes of two operands (+9 %),
+// the next splat's coefficients loaded ahead (+9 %), the next batch's records
+// prefetched into L1 (+8 %).
+constexpr float BWD_BAND = 4e-6f;
+constexpr int BWD_GRP = 8;
+constexpr int BWD_BATCH = 64;
+
+template <int TW, int TH, bool RECT, int PPT, bool STORE = false>
+__global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 10) k_blend_bwd(BlendArgs a) {
     constexpr int NT = TW * TH / PPT;
-    constexpr int NACC = 9;
-    // pairs of pixels in packed f32x2 lanes (the store-all study keeps the
-    // scalar loop)
-    constexpr bool PACKB = PPT % 2 == 0 && !STORE;
-    const float2 one2 = make_float2(a.one, a.one);
-    __shared__ float4 s_a[BATCH];
-    __shared__ float4 s_c[BATCH];
-    __shared__ float4 s_k[BATCH];
-    __shared__ int s_li[BATCH];
-    __shared__ uint8_t s_wm[BATCH];
-    __shared__ uint32_t s_slot[BATCH];
-    __shared__ float s_acc[BATCH][NACC];
-    __shared__ int s_wsum[NT / 32];
+    constexpr int NW = NT / 32;
+    constexpr int H = PPT / 2;
+    constexpr float LOG2E = 1.44269504f;
+    constexpr float L255 = 7.99435344f;    // log2(255)
+    constexpr float L099 = -0.0144995697f;  // log2(0.99)
+    __shared__ float4 s_a[BWD_BATCH];  // sx, sy, log2(opacity), opacity
+    __shared__ float4 s_c[BWD_BATCH];  // a, b, c, largest p decided without the exact arithmetic
+    __shared__ float4 s_k[BWD_BATCH];  // colour, power floor
+    __shared__ uint2 s_r[RECT ? BWD_BATCH : 1];
+    __shared__ uint32_t s_slot[BWD_BATCH];
+    __shared__ uint8_t s_wm[BWD_BATCH];
+    __shared__ float4 s_b4[NW][BWD_GRP][32];
+    __shared__ float2 s_b2[NW][BWD_GRP][32];
     __shared__ int s_tile;
     __shared__ int s_maxlc;
     constexpr int RW = (32 / TW) * PPT;  // pixel rows per warp
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t wbit = 1u << (tid >> 5);
+    const float2 one2 = make_float2(a.one, a.one);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int total_tiles = a.total_tiles ? (int)*a.total_tiles : a.total_tiles_host;
     const size_t S = (size_t)a.n_per_view * a.nviews;
     for (;;) {
@@ -414,226 +409,231 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 8 : PPT == 4 ? 12 : 
         const int px = tx * TW + (tid % TW), py0 = ty * TH + (tid / TW) * PPT;
         const float pxf = (float)px + 0.5f;
         const float x0c = (float)(tx * TW) + 0.5f, x1c = (float)(min(tx * TW + TW, c.width) - 1) + 0.5f;
-        const float y0c = (float)(ty * TH) + 0.5f, y1c = (float)(min(ty * TH + TH, c.height) - 1) + 0.5f;
         const uint2 rg = a.ranges[tile];
         int lc[PPT];
-        float T[PPT], dl0[PPT], dl1[PPT], dl2[PPT], sbe[PPT], pyc[PPT];
+        float2 T[H], d0[H], d1[H], d2[H], nsb[H], pyc[H];
         int my_maxlc = -1;
 #pragma unroll
-        for (int p = 0; p < PPT; ++p) {
-            const int py = py0 + p;
-            pyc[p] = (float)py + 0.5f;
-            lc[p] = -1;
-            T[p] = 0.0f;
-            dl0[p] = dl1[p] = dl2[p] = 0.0f;
-            if (px < c.width && py < c.height) {
-                size_t pix = (size_t)c.pix_base + (size_t)py * c.width + px;
-                lc[p] = a.last[pix];
-                T[p] = a.final_t[pix];
-                dl0[p] = a.dl[pix * 3 + 0];
-                dl1[p] = a.dl[pix * 3 + 1];
-                dl2[p] = a.dl[pix * 3 + 2];
+        for (int h = 0; h < H; ++h) {
+            float t[2], e0[2], e1[2], e2[2], sb[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int py = py0 + 2 * h + j;
+                int l = -1;
+                t[j] = e0[j] = e1[j] = e2[j] = 0.0f;
+                if (px < c.width && py < c.height) {
+                    const size_t pix = (size_t)c.pix_base + (size_t)py * c.width + px;
+                    l = a.last[pix];
+                    t[j] = a.final_t[pix];
+                    e0[j] = a.dl[pix * 3 + 0];
+                    e1[j] = a.dl[pix * 3 + 1];
+                    e2[j] = a.dl[pix * 3 + 2];
+                }
+                // dL/dpixel . (colour behind the current splat), behind = T_final * bg
+                sb[j] = __fmaf_rn(e2[j], t[j] * a.bg[2], __fmaf_rn(e1[j], t[j] * a.bg[1], e0[j] * (t[j] * a.bg[0])));
+                lc[2 * h + j] = l;
+                my_maxlc = max(my_maxlc, l);
             }
-            // dL/dpixel . (colour behind the current splat), behind = T_final * bg
-            sbe[p] = __fmaf_rn(dl2[p], T[p] * a.bg[2], __fmaf_rn(dl1[p], T[p] * a.bg[1], dl0[p] * (T[p] * a.bg[0])));
-            my_maxlc = max(my_maxlc, lc[p]);
+            T[h] = make_float2(t[0], t[1]);
+            d0[h] = make_float2(e0[0], e0[1]);
+            d1[h] = make_float2(e1[0], e1[1]);
+            d2[h] = make_float2(e2[0], e2[1]);
+            nsb[h] = make_float2(-sb[0], -sb[1]);
+            pyc[h] = make_float2((float)(py0 + 2 * h) + 0.5f, (float)(py0 + 2 * h) + 1.5f);
         }
         const int warp_maxlc = __reduce_max_sync(0xffffffffu, my_maxlc);
         if (lane == 0 && warp_maxlc >= 0) atomicMax(&s_maxlc, warp_maxlc);
         __syncthreads();
         const int maxlc = s_maxlc;
-        for (int hi = maxlc; hi >= 0; hi -= BATCH) {
-            const int lo = max(hi - BATCH + 1, 0);
-            const int nb = stage_batch<NT, BATCH, RW, true>(a, S, rg.x + (uint32_t)lo, rg.x + (uint32_t)hi + 1u, lo, x0c, x1c, y0c,
-                                                      y1c, ty * TH, c.height, s_a, s_c, s_k, s_li, s_wm, s_slot, s_wsum, nullptr);
-            for (int k = tid; k < nb; k += NT) {
+        for (int hi_li = maxlc; hi_li >= 0; hi_li -= BWD_BATCH) {
+            const int lo = max(hi_li - BWD_BATCH + 1, 0);
+            // ---- stage list entries [lo, hi_li], each with the mask of the warps
+            // whose strip of pixel rows it can reach
+            for (int j = tid; j < BWD_BATCH; j += NT) {
+                uint32_t wm = 0;
+                if (lo + j <= hi_li) {
+                    const uint32_t slot = a.pair_vals[rg.x + (uint32_t)(lo + j)];
+                    const float4 A = a.rec[slot];
+                    const float4 Q = a.rec[S + slot];
+                    const float4 K = a.rec[2 * S + slot];
+                    const float thr = power_floor(A.z);
+                    const TileTest t = tile_test_setup(A.x, A.y, Q.x, Q.y, Q.z, thr);
 #pragma unroll
-                for (int q = 0; q < NACC; ++q) s_acc[k][q] = 0.0f;
+                    for (int ww = 0; ww < NW; ++ww) {
+                        const int r0 = ty * TH + ww * RW;
+                        if (r0 >= c.height) continue;
+                        const float sy0 = (float)r0 + 0.5f, sy1 = (float)(min(r0 + RW, c.height) - 1) + 0.5f;
+                        if (!tile_rejects(t, x0c, x1c, sy0, sy1)) wm |= 1u << ww;
+                    }
+                    if (wm) {
+                        const float lop = log2f(A.z);
+                        s_a[j] = make_float4(A.x, A.y, lop, A.z);
+                        // a conic or colour outside any sane range (NaN and inf among
+                        // them) sends every pixel to the exact arithmetic
+                        const float mag = fabsf(Q.x) + fabsf(Q.y) + fabsf(Q.z) + fabsf(K.x) + fabsf(K.y) + fabsf(K.z);
+                        s_c[j] = make_float4(Q.x, Q.y, Q.z, mag <= 1e25f ? fminf(L099, lop) - BWD_BAND : __int_as_float(0x7fc00000));
+                        s_k[j] = make_float4(K.x, K.y, K.z, thr);
+                        s_slot[j] = slot;
+                        if (RECT) s_r[j] = make_uint2(__float_as_uint(Q.w), __float_as_uint(K.w));
+                    }
+                }
+                s_wm[j] = (uint8_t)wm;
             }
             __syncthreads();
-            for (int k = nb - 1; k >= 0; --k) {
-                const int li = s_li[k];
-                if (li > warp_maxlc || !(s_wm[k] & wbit)) continue;  // warp-uniform
-                float g[NACC];
+            // ---- this warp's entries, back to front
+            int cnt = 0, my_k = 0;
+            auto flush = [&]() {
+                __syncwarp();
+                const int g = lane & (BWD_GRP - 1), q = lane / BWD_GRP;
+                const float4 ctr = s_a[my_k], cq = s_c[my_k];
+                const uint32_t slot = s_slot[my_k];
+                float dx = ((float)(tx * TW + (q * 8) % TW) + 0.5f) - ctr.x;
+                float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, u0 = 0.0f, u1 = 0.0f, u2 = 0.0f, w0 = 0.0f, w1 = 0.0f, w2 = 0.0f;
 #pragma unroll
-                for (int q = 0; q < NACC; ++q) g[q] = 0.0f;
-                bool contrib = false;
-                if (li <= my_maxlc) {
+                for (int e = 0; e < 8; ++e) {
+                    const int l = (q * 8 + e) ^ g;
+                    const float4 f = s_b4[warp][g][l];
+                    const float2 f2 = s_b2[warp][g][l];
+                    c0 += f.x;
+                    c1 += f.y;
+                    c2 += f.z;
+                    const float du = dx * f.w;
+                    u0 += f.w;
+                    u1 += du;
+                    u2 = __fmaf_rn(du, dx, u2);
+                    w0 += f2.x;
+                    w1 = __fmaf_rn(dx, f2.x, w1);
+                    w2 += f2.y;
+                    dx += 1.0f;
+                }
+#pragma unroll
+                for (int o = BWD_GRP; o < 32; o <<= 1) {
+                    c0 += __shfl_xor_sync(0xffffffffu, c0, o);
+                    c1 += __shfl_xor_sync(0xffffffffu, c1, o);
+                    c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+                    u0 += __shfl_xor_sync(0xffffffffu, u0, o);
+                    u1 += __shfl_xor_sync(0xffffffffu, u1, o);
+                    u2 += __shfl_xor_sync(0xffffffffu, u2, o);
+                    w0 += __shfl_xor_sync(0xffffffffu, w0, o);
+                    w1 += __shfl_xor_sync(0xffffffffu, w1, o);
+                    w2 += __shfl_xor_sync(0xffffffffu, w2, o);
+                }
+                // the sums are of negated terms
+                if (g < cnt) {
+                    if (q == 0) red_add_v4(a.acc + slot, -c0, -c1, -c2, -u0 / ctr.w);
+                    if (q == 1) red_add_v4(a.acc + S + slot, 0.5f * u2, w1, 0.5f * w2, -__fmaf_rn(cq.y, w0, cq.x * u1));
+                    if (q == 2) red_add_v4(a.acc + 2 * S + slot, -__fmaf_rn(cq.z, w0, cq.y * u1), 0.0f, 0.0f, 0.0f);
+                }
+                __syncwarp();
+                cnt = 0;
+            };
+#pragma unroll 1
+            for (int half = BWD_BATCH / 32 - 1; half >= 0; --half) {
+                const int kk = half * 32 + lane;
+                unsigned todo = __ballot_sync(0xffffffffu, ((s_wm[kk] >> warp) & 1u) && lo + kk <= warp_maxlc);
+                while (todo) {
+                    const int b = 31 - __clz(todo);
+                    todo ^= 1u << b;
+                    const int k = half * 32 + b;
+                    const int li = lo + k;
                     const float4 A = s_a[k];
                     const float4 Q = s_c[k];
-                    const float4 K = s_k[k];
                     const float dx = pxf - A.x;
                     const float tdx = Q.x * dx * dx;
                     const float t2b = 2.0f * Q.y * dx;
-                    // per-entry factors of the conic / mean gradients
-                    const float hdxx = -0.5f * dx * dx, qxdx = Q.x * dx, qydx = Q.y * dx;
-                    float su = 0.0f, sud = 0.0f, sudd = 0.0f;  // sums over pixels of u, u dy, u dy^2
-                    if (PACKB) {
-                        // pixel pairs (p, p + 1) in packed f32x2 lanes; the power, and
-                        // with it every decision, is rounded per lane exactly as the
-                        // forward rounds it. A lane that does not take this splat
-                        // keeps its T and behind-colour sum and adds zeros.
-                        float2 G0 = bc2(0.0f), G1 = bc2(0.0f), G2 = bc2(0.0f), G3 = bc2(0.0f);
-                        float2 SU = bc2(0.0f), SUD = bc2(0.0f), SUDD = bc2(0.0f);
+                    float2 dy[H], nal[H], um[H];
+                    bool any = false, sure = true;
 #pragma unroll
-                        for (int h = 0; h < PPT / 2; ++h) {
-                            const int p0 = 2 * h, p1 = 2 * h + 1;
-                            bool a0 = li <= lc[p0], a1 = li <= lc[p1];
+                    for (int h = 0; h < H; ++h) {
+                        dy[h] = __fadd2_rn(pyc[h], bc2(-A.y));
+                        // -2 power = (tdx + t2b dy) + (c dy) dy
+                        const float2 s1 = __ffma2_rn(__fmul2_rn(bc2(t2b), dy[h]), one2, bc2(tdx));
+                        const float2 s2 = __ffma2_rn(__fmul2_rn(__fmul2_rn(bc2(Q.z), dy[h]), dy[h]), one2, s1);
+                        const float2 p = __ffma2_rn(s2, bc2(-0.5f * LOG2E), bc2(A.z));
+                        const float2 d = __fadd2_rn(p, bc2(L255));
+                        bool a0 = li <= lc[2 * h], a1 = li <= lc[2 * h + 1];
+                        if (RECT) {
+                            const uint2 r = s_r[k];
+                            a0 = a0 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h);
+                            a1 = a1 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h + 1);
+                        }
+                        sure = sure && fminf(fabsf(d.x), fabsf(d.y)) >= BWD_BAND && fmaxf(p.x, p.y) <= Q.w;
+                        a0 = a0 && d.x > 0.0f;
+                        a1 = a1 && d.y > 0.0f;
+                        any = any || a0 || a1;
+                        const float e0 = ex2_sfu(p.x), e1 = ex2_sfu(p.y);
+                        nal[h] = make_float2(a0 ? -e0 : 0.0f, a1 ? -e1 : 0.0f);
+                        um[h] = nal[h];
+                    }
+                    float4 K = s_k[k];
+                    if (!sure) {
+                        const float4 q = make_float4(Q.x, Q.y, Q.z, A.w);
+#pragma unroll
+                        for (int h = 0; h < H; ++h) {
+                            const float2 zero = make_float2(0.0f, 0.0f);
+                            bool a0 = li <= lc[2 * h], a1 = li <= lc[2 * h + 1];
                             if (RECT) {
-                                a0 = a0 && in_rect(Q.w, K.w, px, py0 + p0);
-                                a1 = a1 && in_rect(Q.w, K.w, px, py0 + p1);
+                                const uint2 r = s_r[k];
+                                a0 = a0 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h);
+                                a1 = a1 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h + 1);
                             }
-                            if (!(a0 || a1)) continue;
-                            const float2 dy2 = __fadd2_rn(make_float2(pyc[p0], pyc[p1]), bc2(-A.y));
-                            const float2 qdd2 = __fmul2_rn(__fmul2_rn(bc2(Q.z), dy2), dy2);
-                            const float2 s1 = __ffma2_rn(__fmul2_rn(bc2(t2b), dy2), one2, bc2(tdx));
-                            const float2 pw = __fmul2_rn(__ffma2_rn(qdd2, one2, s1), bc2(-0.5f));
-                            a0 = a0 && !(pw.x > 0.0f) && !(pw.x < A.w);
-                            a1 = a1 && !(pw.y > 0.0f) && !(pw.y < A.w);
-                            if (!(a0 || a1)) continue;
-                            float2 ge = make_float2(exp_sfu_nonpos(pw.x), exp_sfu_nonpos(pw.y));
-                            float2 ar = __fmul2_rn(bc2(A.z), ge);
-                            if (fabsf(ar.x - 1.0f / 255.0f) < SFU_BAND * (1.0f / 255.0f) || fabsf(ar.x - 0.99f) < SFU_BAND * 0.99f) {
-                                ge.x = expf_fast_nonpos(pw.x);
-                                ar.x = A.z * ge.x;
-                            }
-                            if (fabsf(ar.y - 1.0f / 255.0f) < SFU_BAND * (1.0f / 255.0f) || fabsf(ar.y - 0.99f) < SFU_BAND * 0.99f) {
-                                ge.y = expf_fast_nonpos(pw.y);
-                                ar.y = A.z * ge.y;
-                            }
-                            const float al0 = fminf(ar.x, 0.99f), al1 = fminf(ar.y, 0.99f);
-                            a0 = a0 && !(al0 < 1.0f / 255.0f);
-                            a1 = a1 && !(al1 < 1.0f / 255.0f);
-                            if (!(a0 || a1)) continue;
-                            const float2 al = make_float2(a0 ? al0 : 0.0f, a1 ? al1 : 0.0f);
-                            const float2 om = __ffma2_rn(al, bc2(-1.0f), bc2(1.0f));
-                            const float2 inv = make_float2(__fdividef(1.0f, om.x), __fdividef(1.0f, om.y));
-                            // a lane with alpha = 0 has 1 - alpha = 1 and rcp(1) = 1, so its
-                            // T is multiplied by exactly 1
-                            const float2 Tp = __fmul2_rn(make_float2(T[p0], T[p1]), inv);
-                            T[p0] = Tp.x;
-                            T[p1] = Tp.y;
-                            const float2 w = __fmul2_rn(al, Tp);
-                            const float2 d0 = make_float2(dl0[p0], dl0[p1]);
-                            const float2 d1 = make_float2(dl1[p0], dl1[p1]);
-                            const float2 d2 = make_float2(dl2[p0], dl2[p1]);
-                            G0 = __ffma2_rn(d0, w, G0);
-                            G1 = __ffma2_rn(d1, w, G1);
-                            G2 = __ffma2_rn(d2, w, G2);
-                            const float2 dk = __ffma2_rn(d2, bc2(K.z), __ffma2_rn(d1, bc2(K.y), __fmul2_rn(d0, bc2(K.x))));
-                            const float2 sb = make_float2(sbe[p0], sbe[p1]);
-                            const float2 dda = __ffma2_rn(Tp, dk, __fmul2_rn(make_float2(-sb.x, -sb.y), inv));
-                            const float2 sbn = __ffma2_rn(w, dk, sb);
-                            sbe[p0] = sbn.x;
-                            sbe[p1] = sbn.y;
-                            // zero for a lane that does not take the splat or whose raw
-                            // alpha was clamped (backward.rs:459-461)
-                            const float2 draw = make_float2(a0 && !(ar.x > 0.99f) ? dda.x : 0.0f, a1 && !(ar.y > 0.99f) ? dda.y : 0.0f);
-                            // every lane's exp and raw alpha are finite (power <= 0 up to
-                            // rounding), so a zero draw zeroes its terms
-                            G3 = __ffma2_rn(draw, ge, G3);
-                            const float2 u = __fmul2_rn(draw, ar);
-                            SU = __fadd2_rn(SU, u);
-                            SUD = __ffma2_rn(u, dy2, SUD);
-                            SUDD = __ffma2_rn(__fmul2_rn(u, dy2), dy2, SUDD);
-                            contrib = true;
+                            const float2 x0 = a0 ? bwd_exact_pixel(dx, dy[h].x, q, K.w) : zero;
+                            const float2 x1 = a1 ? bwd_exact_pixel(dx, dy[h].y, q, K.w) : zero;
+                            nal[h] = make_float2(x0.x, x1.x);
+                            um[h] = make_float2(x0.y, x1.y);
+                            any = any || x0.x != 0.0f || x1.x != 0.0f;
                         }
-                        if (contrib) {
-                            g[0] = G0.x + G0.y;
-                            g[1] = G1.x + G1.y;
-                            g[2] = G2.x + G2.y;
-                            g[3] = G3.x + G3.y;
-                            su = SU.x + SU.y;
-                            sud = SUD.x + SUD.y;
-                            sudd = SUDD.x + SUDD.y;
-                        }
-                    } else {
+                        // a colour that is not finite reaches no pixel that does not take it
+                        if (!any) K = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                    if (!__any_sync(0xffffffffu, any)) continue;
+                    float2 G0, G1, G2, SU, SUD, SUDD;
 #pragma unroll
-                    for (int p = 0; p < PPT; ++p) {
-                        if (li > lc[p]) continue;
-                        if (RECT && !in_rect(Q.w, K.w, px, py0 + p)) continue;
-                        // alpha exactly as the forward computed it
-                        const float dy = pyc[p] - A.y;
-                        const float power = -0.5f * (tdx + t2b * dy + Q.z * dy * dy);
-                        if (power > 0.0f || power < A.w) continue;
-                        // alpha to ~1e-6 from the SFU exponential; where that cannot
-                        // settle the forward's decisions (alpha >= 1/255, alpha_raw >
-                        // 0.99), the forward's own exp settles them, so the
-                        // contributing set is exactly the forward's
-                        float g_exp = exp_sfu_nonpos(power);
-                        float alpha_raw = A.z * g_exp;
-                        if (fabsf(alpha_raw - 1.0f / 255.0f) < SFU_BAND * (1.0f / 255.0f) ||
-                            fabsf(alpha_raw - 0.99f) < SFU_BAND * 0.99f) {
-                            g_exp = expf_fast_nonpos(power);
-                            alpha_raw = A.z * g_exp;
-                        }
-                        const float alpha = fminf(alpha_raw, 0.99f);
-                        if (alpha < 1.0f / 255.0f) continue;
-                        float inv_1ma;
+                    for (int h = 0; h < H; ++h) {
+                        // a pixel that does not take the splat has alpha = 0: 1 - alpha = 1
+                        // and rcp(1) = 1 leave its T and behind-colour sum as they are, and
+                        // its terms are zero
+                        const float2 om = __fadd2_rn(one2, nal[h]);
+                        float2 inv;
                         if (STORE) {
                             // store-all variant: T before this splat as the forward saw it
-                            T[p] = a.tstore[(size_t)(rg.x + (uint32_t)li) * (TW * TH) + (tid / TW) * PPT * TW + p * TW + tid % TW];
-                            inv_1ma = 1.0f / (1.0f - alpha);
+                            const float* ts = a.tstore + (size_t)(rg.x + (uint32_t)li) * (TW * TH) + ((tid / TW) * PPT + 2 * h) * TW + tid % TW;
+                            if (nal[h].x != 0.0f) T[h].x = ts[0];
+                            if (nal[h].y != 0.0f) T[h].y = ts[TW];
+                            inv = make_float2(1.0f / om.x, 1.0f / om.y);
                         } else {
-                            inv_1ma = __fdividef(1.0f, 1.0f - alpha);
-                            T[p] = T[p] * inv_1ma;
+                            inv = make_float2(rcp_sfu(om.x), rcp_sfu(om.y));
+                            T[h] = __fmul2_rn(T[h], inv);
                         }
-                        // gradient terms of backward.rs:453-484, as fused multiply-adds.
-                        // The colour behind enters only as dL/dpixel . behind, so one
-                        // scalar per pixel (sbe) replaces the three channels; the conic
-                        // and mean terms are linear in u = dL/dpower per pixel, so the
-                        // thread sums u, u dy and u dy^2 over its pixels and forms the
-                        // five terms once per splat (dx is the thread's column).
-                        const float weight = alpha * T[p];
-                        g[0] = __fmaf_rn(dl0[p], weight, g[0]);
-                        g[1] = __fmaf_rn(dl1[p], weight, g[1]);
-                        g[2] = __fmaf_rn(dl2[p], weight, g[2]);
-                        const float dk = __fmaf_rn(dl2[p], K.z, __fmaf_rn(dl1[p], K.y, dl0[p] * K.x));
-                        const float dl_dalpha = __fmaf_rn(T[p], dk, -sbe[p] * inv_1ma);
-                        sbe[p] = __fmaf_rn(weight, dk, sbe[p]);
-                        const float dl_draw = alpha_raw > 0.99f ? 0.0f : dl_dalpha;
-                        g[3] = __fmaf_rn(dl_draw, g_exp, g[3]);
-                        const float u = dl_draw * alpha_raw;
-                        su += u;
-                        sud = __fmaf_rn(u, dy, sud);
-                        sudd = __fmaf_rn(u * dy, dy, sudd);
-                        contrib = true;
-                    }
-                    }
-                    if (contrib) {
-                        g[4] = hdxx * su;
-                        g[5] = -dx * sud;
-                        g[6] = -0.5f * sudd;
-                        g[7] = __fmaf_rn(Q.y, sud, qxdx * su);
-                        g[8] = __fmaf_rn(Q.z, sud, qydx * su);
-                    }
-                }
-                const unsigned cm = __ballot_sync(0xffffffffu, contrib);
-                if (cm != 0u) {
-                    if ((cm & (cm - 1u)) == 0u) {
-                        // a single contributing thread: add its values directly
-                        if (contrib) {
-#pragma unroll
-                            for (int q = 0; q < NACC; ++q) atomicAdd(&s_acc[k][q], g[q]);
+                        const float2 nw = __fmul2_rn(nal[h], T[h]);
+                        const float2 dk = __ffma2_rn(d2[h], bc2(K.z), __ffma2_rn(d1[h], bc2(K.y), __fmul2_rn(d0[h], bc2(K.x))));
+                        const float2 dda = __ffma2_rn(T[h], dk, __fmul2_rn(nsb[h], inv));
+                        nsb[h] = __ffma2_rn(nw, dk, nsb[h]);
+                        const float2 nu = __fmul2_rn(dda, um[h]);
+                        const float2 nud = __fmul2_rn(nu, dy[h]);
+                        if (h == 0) {
+                            G0 = __fmul2_rn(d0[h], nw);
+                            G1 = __fmul2_rn(d1[h], nw);
+                            G2 = __fmul2_rn(d2[h], nw);
+                            SU = nu;
+                            SUD = nud;
+                            SUDD = __fmul2_rn(nud, dy[h]);
+                        } else {
+                            G0 = __ffma2_rn(d0[h], nw, G0);
+                            G1 = __ffma2_rn(d1[h], nw, G1);
+                            G2 = __ffma2_rn(d2[h], nw, G2);
+                            SU = __fadd2_rn(SU, nu);
+                            SUD = __fadd2_rn(SUD, nud);
+                            SUDD = __ffma2_rn(nud, dy[h], SUDD);
                         }
-                    } else {
-                        warp_reduce_scatter9(g, lane, &s_acc[k][0]);
                     }
+                    s_b4[warp][cnt][lane ^ cnt] = make_float4(G0.x + G0.y, G1.x + G1.y, G2.x + G2.y, SU.x + SU.y);
+                    s_b2[warp][cnt][lane ^ cnt] = make_float2(SUD.x + SUD.y, SUDD.x + SUDD.y);
+                    if ((lane & (BWD_GRP - 1)) == cnt) my_k = k;
+                    if (++cnt == BWD_GRP) flush();
                 }
             }
-            __syncthreads();
-            for (int k = tid; k < nb; k += NT) {
-                const float* q = s_acc[k];
-                bool any = false;
-#pragma unroll
-                for (int i = 0; i < NACC; ++i) any |= (q[i] != 0.0f);
-                if (any) {
-                    const uint32_t slot = s_slot[k];
-                    red_add_v4(a.acc + slot, q[0], q[1], q[2], q[3]);
-                    red_add_v4(a.acc + S + slot, q[4], q[5], q[6], q[7]);
-                    red_add_v4(a.acc + 2 * S + slot, q[8], 0.0f, 0.0f, 0.0f);
-                }
-            }
+            if (cnt) flush();
             __syncthreads();
         }
         __syncthreads();  // every thread has read s_tile / s_maxlc before thread 0 rewrites them
@@ -650,7 +650,7 @@ typedef void (*BlendKernel)(BlendArgs);
 template <int TW, int TH, int BATCH, bool RECT>
 static BlendKernel pick(bool fwd, int ppt) {
     if (fwd) return ppt == 1 ? (BlendKernel)k_blend_fwd<TW, TH, BATCH, RECT, 1> : (BlendKernel)k_blend_fwd<TW, TH, BATCH, RECT, 2>;
-    return ppt == 2 ? (BlendKernel)k_blend_bwd<TW, TH, BATCH, RECT, 2> : (BlendKernel)k_blend_bwd<TW, TH, BATCH, RECT, 4>;
+    return ppt == 2 ? (BlendKernel)k_blend_bwd<TW, TH, RECT, 2> : (BlendKernel)k_blend_bwd<TW, TH, RECT, 4>;
 }
 
 template <int TW, int TH, bool RECT>
@@ -766,7 +766,7 @@ void launch_blend_backward(const BlendArgs& a, int tw, int th, int batch, cudaSt
 // a.tstore[(list position) * 256 + pixel in tile], the backward reads it back
 // instead of rebuilding T from the final T.
 void launch_blend_store_all(const BlendArgs& a, bool fwd, cudaStream_t st) {
-    BlendKernel k = fwd ? (BlendKernel)k_blend_fwd<16, 16, 256, false, 2, true> : (BlendKernel)k_blend_bwd<16, 16, 256, false, 2, true>;
+    BlendKernel k = fwd ? (BlendKernel)k_blend_fwd<16, 16, 256, false, 2, true> : (BlendKernel)k_blend_bwd<16, 16, false, 2, true>;
     cudaMemsetAsync(a.work, 0, sizeof(uint32_t), st);
     int grid = grid_for(k, 128);
     if (!a.total_tiles) grid = std::min(grid, std::max(a.total_tiles_host, 1));

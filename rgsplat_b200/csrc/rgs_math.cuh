@@ -221,22 +221,24 @@ __device__ __forceinline__ float2 expf_fast_nonpos2(float2 x, float2 one) {
     return __fmul2_rn(p, scale);
 }
 
-// e^x for x in [-8, 0] from the special-function unit's base-2 exponential
-// (PTX ex2.approx.ftz.f32) of x * log2(e): one multiply and one SFU
-// instruction, within a few ulp (relative error below 1e-6 on that range,
-// checked against expf_fast_nonpos by a GPU test). For values that only need
-// to be close, never for a decision that must match the forward pass.
-__device__ __forceinline__ float exp_sfu_nonpos(float x) {
-    const float y = x * 1.44269504f;
+// 2^x and 1 / x from the special-function unit, one instruction each. For
+// values that only need to be close, never for a decision that must match the
+// forward pass.
+__device__ __forceinline__ float ex2_sfu(float x) {
     float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_sfu(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
-// Relative half-width of the band around a threshold inside which an alpha
-// formed with exp_sfu_nonpos cannot decide which side the forward's exact
-// alpha lies on (4x the tested error bound of exp_sfu_nonpos).
-constexpr float SFU_BAND = 4e-6f;
+// e^x for x in [-8, 0] as ex2_sfu(x * log2(e)), within a few ulp (relative
+// error below 1e-6 on that range, checked against expf_fast_nonpos by a GPU
+// test): the error of the alphas the backward blend forms with ex2_sfu.
+__device__ __forceinline__ float exp_sfu_nonpos(float x) { return ex2_sfu(x * 1.44269504f); }
 
 // Rust f32::max / f32::min ignore a NaN operand (fmaxf/fminf do the same);
 // f32::clamp propagates NaN.
