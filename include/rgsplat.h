@@ -96,13 +96,14 @@ typedef struct rgs_adam_state {
 typedef struct rgs_options {
     int device;           /* CUDA device ordinal (default 0) */
     int tile_w, tile_h;   /* CTA tile: 16x16 (default), 8x32 or 32x8 */
-    int batch;            /* splats staged per shared-memory round: 128, 256 (default), 512 */
+    int batch;            /* 128, 256 (default) or 512: accepted for existing callers; the blend
+                             kernels stage one splat per thread whatever it says */
     int reference_compat; /* 1 (default): keep the reference's Adam quirks (moments are not
                              compacted on prune, optimizer.rs:97-105; "SH DC" lr applies to
                              flat indices 11..13, optimizer.rs:181). 0: moments follow their
                              Gaussians and lr_sh_dc applies to sh[0], sh[16], sh[32]. */
-    int pixels_per_thread; /* forward blend: 1 or 2 (default) vertically adjacent pixels per
-                              thread; the backward blend takes twice as many */
+    int pixels_per_thread; /* 1: the blend kernels run two pixels per thread; 2 (default): four,
+                              or two where a launch has few tiles per SM */
     uint64_t batch_pair_limit; /* pair budget of one batched launch: a batched step whose
                                   (Gaussian, tile) pairs outgrow the pair buffer and pass this
                                   runs as consecutive view groups within it (gradients summed

@@ -642,10 +642,10 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
         }
         CK(cudaEventRecord(study->ev[0], st));
         if (study->store_all) launch_blend_store_all(fa, true, st);
-        else launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        else launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, st);
         CK(cudaEventRecord(study->ev[1], st));
     } else {
-        launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, st);
     }
     mark(ctx, 6);
     CK(cudaGetLastError());
@@ -667,10 +667,10 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
         ba.tstore = fa.tstore;
         CK(cudaEventRecord(study->ev[2], st));
         if (study->store_all) launch_blend_store_all(ba, false, st);
-        else launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        else launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, st);
         CK(cudaEventRecord(study->ev[3], st));
     } else {
-        launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, st);
     }
     mark(ctx, 8);
     launch_geometry(s.params.as<float4>(), s.n, s.cap, cams_dev, 1, ctx->cnt.as<uint32_t>(), ctx->acc.as<float4>(),
@@ -1178,7 +1178,7 @@ int rgs_gpu_render(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_cam
     BlendArgs fa = blend_args(ctx, s, cams_dev, 1, nullptr, tiles, b, bg, true);
     fa.rect_filter = 1;
     fa.empty_tile_black = 0;
-    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, ctx->st);
+    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(rgb_out, ctx->rgb.p, px * 12, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
@@ -1469,7 +1469,7 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
     int rc = bin_batch(ctx, s, cams_dev, V, tiles_cap, false, b, true, zero_bg(bg), st_view_max * (size_t)V);
     if (!rc) {
         BlendArgs fa = blend_args(ctx, s, cams_dev, V, &hd->total_tiles, tiles_cap, b, bg, true);
-        launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, st);
         mark(ctx, 6);
         // the step's targets were copied from host memory on copy_st, issued
         // just before this graph's launch; only the loss waits for them
@@ -1481,7 +1481,7 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
         mark(ctx, 7);
         cudaMemsetAsync(ctx->acc.p, 0, std::max<size_t>(S, 1) * 3 * sizeof(float4), st);
         BlendArgs ba = blend_args(ctx, s, cams_dev, V, &hd->total_tiles, tiles_cap, b, bg, false);
-        launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, st);
+        launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, st);
         mark(ctx, 8);
         if (fused) {
             AdamArgs a;
@@ -2222,7 +2222,7 @@ int rgs_debug_forward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_
     size_t px, tiles, lb;
     if ((rc = debug_bin(ctx, gaussians, n, camera, dc, &cams_dev, b, px, tiles, lb))) return rc;
     BlendArgs fa = blend_args(ctx, ctx->sc, cams_dev, 1, nullptr, tiles, b, bg, true);
-    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, ctx->st);
+    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(rgb, ctx->rgb.p, px * 12, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(final_t, ctx->final_t.p, px * 4, cudaMemcpyDeviceToHost, ctx->st));
@@ -2245,13 +2245,13 @@ int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs
     dc.target = ctx->target_stage.as<float>();
     if ((rc = upload_single_cam(ctx, dc, &cams_dev))) return rc;
     BlendArgs fa = blend_args(ctx, ctx->sc, cams_dev, 1, nullptr, tiles, b, bg, true);
-    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, ctx->st);
+    launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
     float* losses_dev = (float*)((char*)ctx->outd.p + offsetof(StepOut, losses));
     CK(launch_loss(cams_dev, 1, (int)lb, ctx->rgb.as<float>(), lambda, ctx->dl.as<float>(), ctx->partials.as<float>(),
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, ctx->st));
     CK(cudaMemsetAsync(ctx->acc.p, 0, std::max<size_t>(n, 1) * 3 * sizeof(float4), ctx->st));
     BlendArgs ba = blend_args(ctx, ctx->sc, cams_dev, 1, nullptr, tiles, b, bg, false);
-    launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, ctx->opt.batch, ctx->st);
+    launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
     CK(cudaGetLastError());
     if (n) {
         std::vector<float4> acc(3 * n);

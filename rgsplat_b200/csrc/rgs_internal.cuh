@@ -267,7 +267,7 @@ struct BlendArgs {
     uint32_t* work;                // dynamic tile counter (zeroed by the launcher)
     int rect_filter;               // per-pixel reference-tile membership test
     int empty_tile_black;          // pixels of empty reference tiles render 0, not bg
-    int pixels_per_thread;         // 1 or 2 vertically adjacent pixels per thread
+    int pixels_per_thread;         // 1: two pixels per thread; 2: four, or two where tiles are few
     float* tstore;                 // store-all variant only: T per (list position, tile pixel)
     int bg_start;                  // preview compositing (rasterizer.rs:133): colour starts at bg and
                                    // the output is that sum, bg not scaled by the final T
@@ -275,8 +275,8 @@ struct BlendArgs {
                                    // products as fma(product, one, acc) so that the code
                                    // generator cannot fuse the multiply into the add
 };
-void launch_blend_forward(const BlendArgs& a, int tile_w, int tile_h, int batch, cudaStream_t st);
-void launch_blend_backward(const BlendArgs& a, int tile_w, int tile_h, int batch, cudaStream_t st);
+void launch_blend_forward(const BlendArgs& a, int tile_w, int tile_h, cudaStream_t st);
+void launch_blend_backward(const BlendArgs& a, int tile_w, int tile_h, cudaStream_t st);
 void launch_blend_store_all(const BlendArgs& a, bool fwd, cudaStream_t st);
 // Largest relative difference of the backward's SFU exponential from the
 // forward's exp over n points on [lo, hi] (float bits, atomicMax into *out).

@@ -188,37 +188,39 @@ __device__ __forceinline__ float expf_fast_nonpos(float x) {
 // rounds once, exactly like the separate add.
 __device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
 
-// expf_fast_nonpos on two lanes: the same operations in the same order per
-// lane (a negated operand moves to the exactly representable constant), so
-// each lane is bit-identical to the scalar routine. 2^k is assembled from the
-// shifted sum j, whose low mantissa bits hold k (bits(j) = bits(SHIFT) + k),
-// which is the same power of two the scalar routine builds from (int)k.
-__device__ __forceinline__ float2 expf_fast_nonpos2(float2 x, float2 one) {
+// expf_fast_nonpos(-y / 2) on two lanes (y = -2 power, as the blend has it): the
+// same operations in the same order per lane, with every power of two moved
+// into the exactly representable constants (r = -2 rh is kept in place of rh,
+// and the polynomial's step i carries a factor (-1/2)^i / 4), so each lane is
+// bit-identical to the scalar routine. The final 2^k is an addition to the
+// exponent field: the low mantissa bits of the shifted sum j hold k (bits(j) =
+// bits(SHIFT) + k, and bits(SHIFT) << 23 is 0 mod 2^32), and p is in
+// [0.7, 1.42], so the sum is the product whenever it is a normal number.
+__device__ __forceinline__ float2 expf_fast_neghalf2(float2 y, float2 one) {
     const float L2E = 1.44269502f;
     const float SHIFT = 12582912.0f;
     const float LN2_HI = 0.693145751953125f;
     const float LN2_LO = 1.42860677e-06f;
-    const float2 j = __ffma2_rn(x, bc2(L2E), bc2(SHIFT));
+    const float2 j = __ffma2_rn(y, bc2(-0.5f * L2E), bc2(SHIFT));
     const float2 k = __fadd2_rn(j, bc2(-SHIFT));
-    const float2 rh = __ffma2_rn(k, bc2(-LN2_HI), x);
+    const float2 r = __ffma2_rn(k, bc2(2.0f * LN2_HI), y);
     const float2 rl = __fmul2_rn(k, bc2(-LN2_LO));
-    float2 q = __ffma2_rn(bc2(2.48015873e-05f), rh, bc2(1.98412698e-4f));
-    q = __ffma2_rn(q, rh, bc2(1.38888889e-3f));
-    q = __ffma2_rn(q, rh, bc2(8.33333333e-3f));
-    q = __ffma2_rn(q, rh, bc2(4.16666667e-2f));
-    q = __ffma2_rn(q, rh, bc2(1.66666667e-1f));
-    q = __ffma2_rn(q, rh, bc2(0.5f));
-    const float2 hi = __fadd2_rn(one, rh);
+    float2 q = __ffma2_rn(bc2(2.48015873e-05f / 256.0f), r, bc2(1.98412698e-4f / -128.0f));
+    q = __ffma2_rn(q, r, bc2(1.38888889e-3f / 64.0f));
+    q = __ffma2_rn(q, r, bc2(8.33333333e-3f / -32.0f));
+    q = __ffma2_rn(q, r, bc2(4.16666667e-2f / 16.0f));
+    q = __ffma2_rn(q, r, bc2(1.66666667e-1f / -8.0f));
+    q = __ffma2_rn(q, r, bc2(0.5f / 4.0f));
+    const float2 hi = __ffma2_rn(r, bc2(-0.5f), one);                      // 1 + rh
     const float2 omh = __ffma2_rn(hi, make_float2(-one.x, -one.y), one);  // 1 - hi, rounded once
-    const float2 lo = __fadd2_rn(omh, rh);
-    const float2 s = __fmul2_rn(rh, rh);
+    const float2 lo = __ffma2_rn(r, bc2(-0.5f), omh);                     // omh + rh
+    const float2 s = __fmul2_rn(r, r);                                    // 4 rh^2
     float2 tail = __ffma2_rn(s, q, lo);
     const float2 ea = __fadd2_rn(hi, tail);
     tail = __ffma2_rn(rl, ea, tail);
     const float2 p = __fadd2_rn(hi, tail);
-    const float2 scale = make_float2(__int_as_float((__float_as_int(j.x) - 0x4B3FFF81) << 23),
-                                     __int_as_float((__float_as_int(j.y) - 0x4B3FFF81) << 23));
-    return __fmul2_rn(p, scale);
+    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(j.x) << 23)),
+                       __int_as_float(__float_as_int(p.y) + (__float_as_int(j.y) << 23)));
 }
 
 // 2^x and 1 / x from the special-function unit, one instruction each. For
