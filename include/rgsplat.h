@@ -362,7 +362,8 @@ typedef struct rgs_stats {
                                when its pairs passed 2^30 (each group within it) */
     uint32_t reserved;
     uint64_t supertile_entries; /* (supertile, splat) entries binned: each splat once
-                                   per 4x4-tile supertile its tile rectangle meets */
+                                   per 4x4-tile supertile its tile rectangle meets (with a
+                                   zero background, its reachable span of each row) */
 } rgs_stats;
 int rgs_get_stats(rgs_ctx* ctx, rgs_stats* out);
 

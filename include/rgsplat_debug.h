@@ -36,6 +36,12 @@ int rgs_debug_tile_lists(rgs_ctx* ctx, const float* gaussians, size_t n, const r
 int rgs_debug_pruned_tile_lists(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera* camera,
                                 uint64_t* n_pairs, int32_t* offsets, int32_t* entries, size_t cap);
 
+/* The binning keeps an entry's 16-tile mask in the upper half of its sort key
+ * where every supertile id of the batch fits 16 bits, and forms the masks after
+ * the sort otherwise (batches over 65536 supertiles of 4x4 tiles). on != 0 makes
+ * this context use the second form at any size; the lists are the same. */
+int rgs_debug_wide_supertiles(rgs_ctx* ctx, int on);
+
 /* forward_pass caches (backward.rs:296-385): rgb w*h*3, final T w*h, last
  * contributor (index into the pixel's tile list, -1 if none) w*h. */
 int rgs_debug_forward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera* camera, const float bg[3],

@@ -221,6 +221,7 @@ SIGNATURES = {
                                        C.POINTER(C.c_int32), C.c_size_t]),
     "rgs_debug_pruned_tile_lists": (C.c_int, [CTX, FP, C.c_size_t, C.POINTER(rgs_camera), C.POINTER(C.c_uint64),
                                               C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.c_size_t]),
+    "rgs_debug_wide_supertiles": (C.c_int, [CTX, C.c_int]),
     "rgs_debug_forward": (C.c_int, [CTX, FP, C.c_size_t, C.POINTER(rgs_camera), FP, FP, FP, C.POINTER(C.c_int32)]),
     "rgs_debug_backward": (C.c_int, [CTX, FP, C.c_size_t, C.POINTER(rgs_camera), FP, FP, C.c_float, FP, FP]),
     "rgs_debug_trainer_batch_pixels": (C.c_int, [CTX, C.c_size_t, FP, FP, FP]),

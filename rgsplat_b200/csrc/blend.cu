@@ -704,7 +704,6 @@ static void launch(const BlendArgs& a, int tw, int th, bool fwd, cudaStream_t st
     const int ppt = pixels_for(a, tw, th, rect, fwd);
     BlendKernel k = select_kernel(tw, th, rect, fwd, ppt);
     const int threads = tw * th / ppt;
-    cudaMemsetAsync(a.work, 0, sizeof(uint32_t), st);
     int grid = grid_for(k, threads);
     if (!a.total_tiles) grid = std::min(grid, std::max(a.total_tiles_host, 1));
     k<<<grid, threads, 0, st>>>(a);
@@ -775,7 +774,6 @@ void launch_blend_backward(const BlendArgs& a, int tw, int th, cudaStream_t st) 
 // instead of rebuilding T from the final T.
 void launch_blend_store_all(const BlendArgs& a, bool fwd, cudaStream_t st) {
     BlendKernel k = fwd ? (BlendKernel)k_blend_fwd<16, 16, false, 2, true> : (BlendKernel)k_blend_bwd<16, 16, false, 2, true>;
-    cudaMemsetAsync(a.work, 0, sizeof(uint32_t), st);
     int grid = grid_for(k, 128);
     if (!a.total_tiles) grid = std::min(grid, std::max(a.total_tiles_host, 1));
     k<<<grid, 128, 0, st>>>(a);

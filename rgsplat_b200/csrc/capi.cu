@@ -40,38 +40,43 @@ struct StepHdr {
     DevCam cams[MAX_VIEWS];
 };
 
-struct StepOut {
-    uint32_t pairs;
-    int overflow;
-    uint32_t visible;
-    uint32_t pad;
-    float losses[MAX_VIEWS];
-    unsigned long long pairs64;  // exact pair count (pairs saturates at 2^32 - 1)
-    unsigned long long st_pairs64;  // (supertile, slot) entries of the batch
-    int sort_fault;
-    int pad2;
-};
-
 // Default of rgs_options.batch_pair_limit: a batched step whose (Gaussian,
 // tile) pairs exceed it runs as consecutive view groups that each stay
 // within it (pair buffers and sort scratch take 16 bytes per pair: 17 GB).
 constexpr unsigned long long BATCH_PAIR_LIMIT = 1ull << 30;
 
+// Words of the context's scalar buffer; one copy reads a step's results back.
 enum {
-    SC_PAIRS = 0,
-    SC_OVERFLOW = 2,
-    SC_WORK_F = 3,
+    // zeroed at the start of every binning
+    SC_OVERFLOW = 0,
+    SC_WORK_F = 1,      // dynamic tile counters of the blend kernels
+    SC_PAIRS64 = 2,     // u64: (tile, slot) pairs
     SC_WORK_B = 4,
+    SC_ZEROED = 5,
     SC_FINITE = 5,
-    SC_VISIBLE = 6,
-    SC_FAULT = 7,    // sticky: a sort pass's staged copies timed out
-    SC_PAIRS64 = 8,  // u64 over slots 8 and 9
-    SC_NVIS64 = 10,  // u64 over slots 10 and 11: slots with tile pairs
-    SC_NVIS = 12,    // the same, u32 (the depth sort's element count)
-    SC_STPAIRS64 = 14,  // u64 over 14 and 15: (supertile, slot) entries
-    SC_STPAIRS = 16,    // the same, saturated u32
-    SC_STEFF = 17,      // entries held (the supertile sort's element count)
-    SC_COUNT = 18
+    SC_FAULT = 6,       // sticky: a sort pass's staged copies timed out
+    SC_STEFF = 7,       // entries held (the supertile sort's element count)
+    SC_NVIS64 = 8,      // u64: slots with tile pairs
+    SC_STPAIRS64 = 10,  // u64: (supertile, slot) entries
+    SC_NVIS = 12,       // the same two as u32 (the latter saturated)
+    SC_STPAIRS = 13,
+    SC_LOSSES = 16,     // f32 per view
+    SC_COUNT = 16 + MAX_VIEWS
+};
+
+// The scalar buffer as read back.
+struct StepOut {
+    uint32_t w[SC_COUNT];
+    unsigned long long u64(int i) const {
+        unsigned long long v;
+        std::memcpy(&v, w + i, 8);
+        return v;
+    }
+    float loss(int v) const {
+        float f;
+        std::memcpy(&f, w + SC_LOSSES + v, 4);
+        return f;
+    }
 };
 
 }  // namespace
@@ -90,13 +95,13 @@ struct rgs_ctx {
     DBuf hdr;       // StepHdr (device)
     StepHdr* hdr_h = nullptr;  // pinned
     StepOut* out_h = nullptr;  // pinned
-    DBuf outd;      // StepOut (device)
-    DBuf rec, cnt, tdesc, spans, dkey, ids, acc, gv;
+    DBuf rec, cnt, spans, dkey, acc, gv;
     DBuf ckey, cslot, chunk_counts;  // slots with tile pairs, compacted for the depth sort
-    // supertile binning: per slot the supertile count and rectangle, per
-    // entry the tile mask, per chunk of entries and tile position the counts,
-    // per position the total, and the count scan's block sums
-    DBuf st_cnt, st_desc, st_masks, st_chunks, st_planes, st_block_sums;
+    // supertile binning: per slot the entry count, per entry the tile mask (only where it does not fit the
+    // entry's key), per chunk of entries and tile position the counts, per
+    // position the total, and the entry scan's block sums
+    DBuf st_cnt, st_masks, st_chunks, st_planes, st_block_sums;
+    bool wide_supertiles = false;  // debug: keep the masks out of the keys
     DBuf gcache;  // per-Gaussian view-independent projection terms, [2][cap] float4
     DBuf pkeys, pvals;
     uint32_t pair_cap = 0;
@@ -104,7 +109,7 @@ struct rgs_ctx {
     int batch_views = 0;      // views whose pixels the buffers hold from the last
                               // batched pass run as one group (0: none)
     DBuf ranges, rgb, final_t, last, dl, partials;
-    DBuf scalars, block_sums, view_pairs;
+    DBuf scalars, view_pairs;
     SortScratch sort;
     SfmScratch sfm;
     DBuf dens_scratch, dens_out, m_tmp;
@@ -383,17 +388,14 @@ int ensure_work(rgs_ctx* ctx, size_t S, size_t px, size_t tiles, size_t lblocks,
     CK(ctx->acc.ensure(std::max<size_t>(S, 1) * 3 * sizeof(float4)));
     CK(ctx->gv.ensure(std::max<size_t>(S, 1) * 4 * sizeof(float4)));
     CK(ctx->cnt.ensure(std::max<size_t>(S, 1) * 4));
-    CK(ctx->tdesc.ensure(std::max<size_t>(S, 1) * 8));
     CK(ctx->spans.ensure(std::max<size_t>(S, 1) * 32));
     CK(ctx->dkey.ensure(std::max<size_t>(S, 1) * 4));
-    CK(ctx->ids.ensure(std::max<size_t>(S, 1) * 4));
     CK(ctx->ckey.ensure(std::max<size_t>(S, 1) * 4));
     CK(ctx->cslot.ensure(std::max<size_t>(S, 1) * 4));
     CK(ctx->chunk_counts.ensure(std::max<size_t>(compact_chunks(S), 1) * 8));
     CK(ctx->st_cnt.ensure(std::max<size_t>(S, 1) * 4));
-    CK(ctx->st_desc.ensure(std::max<size_t>(S, 1) * 8));
     CK(ctx->st_planes.ensure(ST_TILES * 4));
-    CK(ctx->st_block_sums.ensure((size_t)bin_grid_blocks() * 8 + 64));
+    CK(ctx->st_block_sums.ensure((size_t)bin_grid_max() * 8 + 64));
     CK(ctx->ranges.ensure(std::max<size_t>(tiles, 1) * sizeof(uint2)));
     CK(ctx->rgb.ensure(px * 3 * 4));
     CK(ctx->final_t.ensure(px * 4));
@@ -401,10 +403,8 @@ int ensure_work(rgs_ctx* ctx, size_t S, size_t px, size_t tiles, size_t lblocks,
     CK(ctx->dl.ensure(px * 3 * 4));
     CK(ctx->partials.ensure(std::max<size_t>(lblocks, 1) * 2 * 4));
     CK(ctx->scalars.ensure(SC_COUNT * 4));
-    CK(ctx->block_sums.ensure((size_t)bin_grid_blocks() * 8 + 64));
     CK(ctx->view_pairs.ensure(MAX_VIEWS * 8));
     CK(ctx->hdr.ensure(sizeof(StepHdr)));
-    CK(ctx->outd.ensure(sizeof(StepOut)));
     (void)V;
     // whatever runs next writes the pixel buffers
     ctx->batch_views = 0;
@@ -429,7 +429,6 @@ int ensure_pairs(rgs_ctx* ctx, unsigned long long K) {
     ctx->st_chunks.release();
     CK(ctx->pkeys.ensure(cap * 4));
     CK(ctx->pvals.ensure(cap * 4));
-    CK(ctx->st_masks.ensure(cap * 2));
     CK(ctx->st_chunks.ensure(supertile_chunks(cap) * ST_TILES * 4));
     ctx->pair_cap = (uint32_t)cap;
     return RGS_OK;
@@ -440,34 +439,54 @@ struct Binned {
     const uint32_t* vals;
 };
 
-// Projection + depth sort + pair emission + tile sort + ranges for one batch.
-// `k_host` >= 0 means the pair count was read back (plain path).
+// Supertiles of any V views of this context (a captured graph is replayed for
+// other view sets).
+size_t supertile_cap(rgs_ctx* ctx, int V) {
+    size_t most = 1;
+    for (const rgs_camera& cam : ctx->cams) {
+        const size_t tx = (cam.width + ctx->opt.tile_w - 1) / ctx->opt.tile_w, ty = (cam.height + ctx->opt.tile_h - 1) / ctx->opt.tile_h;
+        most = std::max(most, ((tx + ST_EDGE - 1) / ST_EDGE) * ((ty + ST_EDGE - 1) / ST_EDGE));
+    }
+    return most * (size_t)V;
+}
+
+// Whether an entry's key has room for its tile mask above the supertile id.
+bool packed_entries(const rgs_ctx* ctx, size_t st_cap) { return st_cap <= 65536 && !ctx->wide_supertiles; }
+
+// Reads the scalar buffer back and waits for the stream.
+int read_scalars(rgs_ctx* ctx) {
+    CK(cudaMemcpyAsync(ctx->out_h, ctx->scalars.p, sizeof(StepOut), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    if (ctx->out_h->w[SC_FAULT]) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
+    return RGS_OK;
+}
+
+// Projection + depth sort + entry emission + supertile sort + tile lists for
+// one batch. host_count: the pair count is read back and the buffers sized for
+// it (plain path).
 // prune: tile lists hold only the (tile, splat) pairs the blend's own tile
 // test keeps (exact: the blend drops the others from every batch anyway).
 // Only valid with a zero background, where a pixel whose reference tile list
 // is empty renders the same 0 as one whose splats all miss it.
 int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tiles, bool host_count, Binned& out,
-              bool project = true, bool prune = false, size_t st_cap = 0) {
+              bool project, bool prune, size_t st_cap = 0) {
     // supertiles the buffers and scans cover: the batch's own unless the
     // caller (a captured graph replayed for other views) gives a bound
     if (!st_cap) st_cap = std::max<size_t>(ctx->hdr_h->total_st, 1);
     cudaStream_t st = ctx->st;
     const size_t S = (size_t)s.n * V;
     uint32_t* sc = ctx->scalars.as<uint32_t>();
-    if (project) {
-        cudaMemsetAsync(sc + SC_VISIBLE, 0, 4, st);
+    cudaMemsetAsync(sc, 0, SC_ZEROED * 4, st);
+    if (project)
         launch_project(s.params.as<float4>(), s.n, s.cap, cams_dev, V, ctx->opt.tile_w, ctx->opt.tile_h,
-                       ctx->rec.as<float4>(), ctx->cnt.as<uint32_t>(), ctx->tdesc.as<uint2>(), ctx->dkey.as<uint32_t>(),
-                       ctx->ids.as<uint32_t>(), prune ? 1 : 0, sc + SC_VISIBLE, ctx->gcache.as<float4>(), ctx->spans.as<uint4>(), st);
-    }
+                       ctx->rec.as<float4>(), ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), prune ? 1 : 0,
+                       ctx->gcache.as<float4>(), ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), st);
     mark(ctx, 1);
     // only the slots with tile pairs go through the depth sort, gathered in
-    // slot order (the stable sort then still breaks depth ties by index);
-    // the gather also writes each slot's supertile rectangle and count
+    // slot order (the stable sort then still breaks depth ties by index)
     launch_compact_visible(ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), (uint32_t)S,
                            ctx->chunk_counts.as<unsigned long long>(), ctx->ckey.as<uint32_t>(), ctx->cslot.as<uint32_t>(),
-                           sc + SC_NVIS, (unsigned long long*)(sc + SC_NVIS64), ctx->tdesc.as<uint2>(), cams_dev,
-                           (uint32_t)s.n, ctx->st_cnt.as<uint32_t>(), ctx->st_desc.as<uint2>(), st);
+                           sc + SC_NVIS, (unsigned long long*)(sc + SC_NVIS64), (unsigned long long*)(sc + SC_PAIRS64), st);
     const uint32_t* nvis = sc + SC_NVIS;
     cudaError_t e;
     int which = radix_sort_pairs(ctx->ckey.as<uint32_t>(), ctx->cslot.as<uint32_t>(), (uint32_t)S, nvis, 32, ctx->sort,
@@ -475,24 +494,30 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
     if (e != cudaSuccess) return cuda_fail(ctx, e, "depth sort");
     mark(ctx, 2);
     const uint32_t* order = which ? ctx->sort.vals2.as<uint32_t>() : ctx->cslot.as<uint32_t>();
-    // (tile, slot) pairs of the batch, and (supertile, slot) entries
-    launch_count_scan(order, ctx->cnt.as<uint32_t>(), (uint32_t)S, nvis, ctx->block_sums.as<unsigned long long>(),
-                      sc + SC_PAIRS, (unsigned long long*)(sc + SC_PAIRS64), bin_grid_blocks(), st);
-    launch_count_scan(order, ctx->st_cnt.as<uint32_t>(), (uint32_t)S, nvis, ctx->st_block_sums.as<unsigned long long>(),
-                      sc + SC_STPAIRS, (unsigned long long*)(sc + SC_STPAIRS64), bin_grid_blocks(), st);
+    EmitArgs ea;
+    ea.order = order;
+    ea.n_order = nvis;
+    ea.spans = ctx->spans.as<uint4>();
+    ea.st_cnt = ctx->st_cnt.as<uint32_t>();
+    ea.rec = ctx->rec.as<float4>();
+    ea.S = (uint32_t)S;
+    ea.cams = cams_dev;
+    ea.n_per_view = (uint32_t)std::max(s.n, 1);
+    ea.tile_w = ctx->opt.tile_w;
+    ea.tile_h = ctx->opt.tile_h;
+    ea.prune = prune ? 1 : 0;
+    ea.packed = packed_entries(ctx, st_cap) ? 1 : 0;
+    ea.block_sums = ctx->st_block_sums.as<unsigned long long>();
+    ea.total = sc + SC_STPAIRS;
+    ea.total64 = (unsigned long long*)(sc + SC_STPAIRS64);
+    launch_entry_scan(ea, bin_grid_blocks(S), st);
     if (host_count) {
-        unsigned long long K = 0, KS = 0;
-        uint32_t vis = 0;
-        int fault = 0;
-        CK(cudaMemcpyAsync(&K, sc + SC_PAIRS64, 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&KS, sc + SC_STPAIRS64, 8, cudaMemcpyDeviceToHost, st));
-        if (project) CK(cudaMemcpyAsync(&vis, sc + SC_VISIBLE, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&fault, sc + SC_FAULT, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (fault) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
-        ctx->stats.visible += vis;
-        int rc = ensure_pairs(ctx, std::max(K, KS));
+        int rc = read_scalars(ctx);
         if (rc) return rc;
+        const unsigned long long K = ctx->out_h->u64(SC_PAIRS64), KS = ctx->out_h->u64(SC_STPAIRS64);
+        if (project) ctx->stats.visible += ctx->out_h->w[SC_NVIS];
+        if ((rc = ensure_pairs(ctx, std::max(K, KS)))) return rc;
+        if (!ea.packed) CK(ctx->st_masks.ensure((size_t)ctx->pair_cap * 2));
         ctx->stats.pairs += K;
         ctx->stats.supertile_entries += KS;
         // the depth order may live in the sort scratch: size it for the
@@ -511,14 +536,16 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
             if (!tmp.empty()) {
                 CK(cudaMemcpyAsync(ctx->sort.vals2.p, tmp.data(), S * 4, cudaMemcpyHostToDevice, st));
                 CK(cudaStreamSynchronize(st));
-                order = ctx->sort.vals2.as<uint32_t>();
+                ea.order = ctx->sort.vals2.as<uint32_t>();
             }
         }
     }
-    CK(cudaMemsetAsync(sc + SC_OVERFLOW, 0, 4, st));
-    launch_emit_supertiles(order, ctx->st_desc.as<uint2>(), (uint32_t)S, nvis, ctx->st_block_sums.as<unsigned long long>(),
-                           ctx->pkeys.as<uint32_t>(), ctx->pvals.as<uint32_t>(), ctx->pair_cap, (int*)(sc + SC_OVERFLOW),
-                           sc + SC_STPAIRS, sc + SC_STEFF, cams_dev, (uint32_t)s.n, bin_grid_blocks(), st);
+    ea.keys = ctx->pkeys.as<uint32_t>();
+    ea.vals = ctx->pvals.as<uint32_t>();
+    ea.cap = ctx->pair_cap;
+    ea.eff = sc + SC_STEFF;
+    ea.overflow = (int*)(sc + SC_OVERFLOW);
+    launch_emit_supertiles(ea, bin_grid_blocks(S), st);
     mark(ctx, 3);
     int which2 = radix_sort_pairs(ctx->pkeys.as<uint32_t>(), ctx->pvals.as<uint32_t>(), ctx->pair_cap, sc + SC_STEFF,
                                   bits_for(std::max<size_t>(st_cap, 2)), ctx->sort, ctx->sort_grid, st, &e);
@@ -535,14 +562,14 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
     sa.ent_key = ent_keys;
     sa.ent_slot = ent_slot;
     sa.n_ent = sc + SC_STEFF;
-    sa.tdesc = ctx->tdesc.as<uint2>();
     sa.spans = ctx->spans.as<uint4>();
     sa.rec = ctx->rec.as<float4>();
     sa.S = (uint32_t)S;
-    sa.n_per_view = (uint32_t)s.n;
+    sa.n_per_view = ea.n_per_view;
     sa.tile_w = ctx->opt.tile_w;
     sa.tile_h = ctx->opt.tile_h;
     sa.prune = prune ? 1 : 0;
+    sa.packed = ea.packed;
     sa.masks = ctx->st_masks.as<uint16_t>();
     sa.chunk_cnt = ctx->st_chunks.as<uint32_t>();
     sa.chunk_stride = (uint32_t)supertile_chunks(ctx->pair_cap);
@@ -591,16 +618,18 @@ bool zero_bg(const float bg[3]) { return bg[0] == 0.0f && bg[1] == 0.0f && bg[2]
 // Uploads one view's camera header (plain path) and returns its device copy.
 int upload_single_cam(rgs_ctx* ctx, const DevCam& d, DevCam** dev) {
     StepHdr* h = ctx->hdr_h;
+    // the page-locked header may still be on its way from the call before
+    CK(cudaStreamSynchronize(ctx->st));
     h->cams[0] = d;
     h->total_tiles = (uint32_t)(d.tiles_x * d.tiles_y);
     h->total_loss_blocks = (uint32_t)(d.loss_bx * ((d.height + LOSS_TILE - 1) / LOSS_TILE));
     h->total_st = (uint32_t)batch_supertiles(&d, 1);
-    CK(cudaMemcpyAsync(ctx->hdr.p, h, sizeof(StepHdr), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(ctx->hdr.p, h, offsetof(StepHdr, cams) + sizeof(DevCam), cudaMemcpyHostToDevice, ctx->st));
     *dev = (DevCam*)((char*)ctx->hdr.p + offsetof(StepHdr, cams));
-    // the host header is reused by the next call: wait for the copy
-    CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
+
+float* losses_of(rgs_ctx* ctx) { return ctx->scalars.as<float>() + SC_LOSSES; }
 
 // Differentiation study (rgs_render_and_backward_variant): which backward,
 // and the blend-kernel times and blend-state bytes it measured.
@@ -650,14 +679,11 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
     mark(ctx, 6);
     CK(cudaGetLastError());
     if (rgb_host) {
-        int fault = 0;
         CK(cudaMemcpyAsync(rgb_host, ctx->rgb.p, px * 3 * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&fault, ctx->sort.fault, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (fault) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
+        if ((rc = read_scalars(ctx))) return rc;
     }
     if (!do_backward) return RGS_OK;
-    float* losses_dev = (float*)((char*)ctx->outd.p + offsetof(StepOut, losses));
+    float* losses_dev = losses_of(ctx);
     CK(launch_loss(cams_dev, 1, (int)lb, ctx->rgb.as<float>(), lambda, ctx->dl.as<float>(), ctx->partials.as<float>(),
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, st));
     mark(ctx, 7);
@@ -679,11 +705,8 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
     mark(ctx, 9);
     CK(cudaGetLastError());
     if (loss_out) {
-        int fault = 0;
-        CK(cudaMemcpyAsync(loss_out, losses_dev, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&fault, ctx->sort.fault, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (fault) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
+        if ((rc = read_scalars(ctx))) return rc;
+        *loss_out = ctx->out_h->loss(0);
         prof_collect(ctx);
     }
     return RGS_OK;
@@ -801,12 +824,11 @@ void rgs_destroy(rgs_ctx* ctx) {
         s->params.release(); s->grads.release(); s->m1.release(); s->m2.release(); s->accum.release(); s->denom.release();
     }
     for (auto& t : ctx->targets) t.release();
-    DBuf* bufs[] = {&ctx->hdr, &ctx->outd, &ctx->rec, &ctx->cnt, &ctx->tdesc, &ctx->spans, &ctx->gcache, &ctx->dkey, &ctx->ids,
-                    &ctx->ckey, &ctx->cslot, &ctx->chunk_counts, &ctx->st_cnt, &ctx->st_desc, &ctx->st_masks,
-                    &ctx->st_chunks, &ctx->st_planes, &ctx->st_block_sums, &ctx->acc, &ctx->gv, &ctx->pkeys,
+    DBuf* bufs[] = {&ctx->hdr, &ctx->rec, &ctx->cnt, &ctx->spans, &ctx->gcache, &ctx->dkey,
+                    &ctx->ckey, &ctx->cslot, &ctx->chunk_counts, &ctx->st_cnt, &ctx->st_masks, &ctx->st_chunks, &ctx->st_planes, &ctx->st_block_sums, &ctx->acc, &ctx->gv, &ctx->pkeys,
                     &ctx->pvals,
                     &ctx->ranges, &ctx->rgb, &ctx->final_t, &ctx->last, &ctx->dl, &ctx->partials, &ctx->scalars,
-                    &ctx->block_sums, &ctx->view_pairs, &ctx->sort.hist, &ctx->sort.keys2, &ctx->sort.vals2, &ctx->dens_scratch,
+                    &ctx->view_pairs, &ctx->sort.hist, &ctx->sort.keys2, &ctx->sort.vals2, &ctx->dens_scratch,
                     &ctx->dens_out, &ctx->m_tmp, &ctx->stage_a, &ctx->stage_b, &ctx->stage_c, &ctx->stage_d,
                     &ctx->target_stage, &ctx->tstore};
     for (DBuf* b : bufs) b->release();
@@ -1025,7 +1047,7 @@ int rgs_photometric_loss_grad(rgs_ctx* ctx, const float* rendered_rgb, const flo
     dc.target = ctx->target_stage.as<float>();
     DevCam* cams_dev;
     if ((rc = upload_single_cam(ctx, dc, &cams_dev))) return rc;
-    float* losses_dev = (float*)((char*)ctx->outd.p + offsetof(StepOut, losses));
+    float* losses_dev = losses_of(ctx);
     CK(launch_loss(cams_dev, 1, (int)lb, ctx->rgb.as<float>(), lambda, ctx->dl.as<float>(), ctx->partials.as<float>(),
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, ctx->st));
     CK(cudaGetLastError());
@@ -1170,11 +1192,10 @@ int rgs_gpu_render(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_cam
     launch_project_wgsl(s.params.as<float4>(), (int)n, s.cap, cams_dev, mode == RGS_PROJECT_CPU_MATH ? 1 : 0,
                         ctx->stage_b.as<float>(), ctx->stage_c.as<uint32_t>(), ctx->st);
     launch_composite_prepare(ctx->stage_b.as<float>(), (int)n, cams_dev, ctx->opt.tile_w, ctx->opt.tile_h,
-                             ctx->rec.as<float4>(), ctx->cnt.as<uint32_t>(), ctx->tdesc.as<uint2>(), ctx->dkey.as<uint32_t>(),
-                             ctx->ids.as<uint32_t>(),
-                             ctx->st);
+                             ctx->rec.as<float4>(), ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), ctx->spans.as<uint4>(),
+                             ctx->st_cnt.as<uint32_t>(), ctx->st);
     Binned b;
-    if ((rc = bin_batch(ctx, s, cams_dev, 1, tiles, true, b, false))) return rc;
+    if ((rc = bin_batch(ctx, s, cams_dev, 1, tiles, true, b, false, false))) return rc;
     BlendArgs fa = blend_args(ctx, s, cams_dev, 1, nullptr, tiles, b, bg, true);
     fa.rect_filter = 1;
     fa.empty_tile_black = 0;
@@ -1452,21 +1473,17 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
     CK(ctx->sort.keys2.ensure(std::max<size_t>(S, ctx->pair_cap) * 4 + 16));
     CK(ctx->sort.vals2.ensure(std::max<size_t>(S, ctx->pair_cap) * 4 + 16));
     CK(ctx->sort.hist.ensure(sort_hist_bytes(ctx->sort_grid)));
+    const size_t st_cap = supertile_cap(ctx, V);
+    if (!packed_entries(ctx, st_cap)) CK(ctx->st_masks.ensure((size_t)ctx->pair_cap * 2));
     StepHdr* hd = ctx->hdr.as<StepHdr>();
     const DevCam* cams_dev = (const DevCam*)((char*)ctx->hdr.p + offsetof(StepHdr, cams));
-    float* losses_dev = (float*)((char*)ctx->outd.p + offsetof(StepOut, losses));
+    float* losses_dev = losses_of(ctx);
     uint32_t* sc = ctx->scalars.as<uint32_t>();
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(ctx->hdr.p, ctx->hdr_h, sizeof(StepHdr), cudaMemcpyHostToDevice, st);
     mark(ctx, 0);
     Binned b;
-    // supertiles of any V views of this context (the graph is replayed for other view sets)
-    size_t st_view_max = 1;
-    for (const rgs_camera& cam : ctx->cams) {
-        const size_t tx = (cam.width + ctx->opt.tile_w - 1) / ctx->opt.tile_w, ty = (cam.height + ctx->opt.tile_h - 1) / ctx->opt.tile_h;
-        st_view_max = std::max(st_view_max, ((tx + ST_EDGE - 1) / ST_EDGE) * ((ty + ST_EDGE - 1) / ST_EDGE));
-    }
-    int rc = bin_batch(ctx, s, cams_dev, V, tiles_cap, false, b, true, zero_bg(bg), st_view_max * (size_t)V);
+    int rc = bin_batch(ctx, s, cams_dev, V, tiles_cap, false, b, true, zero_bg(bg), st_cap);
     if (!rc) {
         BlendArgs fa = blend_args(ctx, s, cams_dev, V, &hd->total_tiles, tiles_cap, b, bg, true);
         launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, st);
@@ -1497,13 +1514,7 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
                             accumulate, st);
         }
         mark(ctx, 9);
-        cudaMemcpyAsync(&ctx->out_h->pairs, sc + SC_PAIRS, 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&ctx->out_h->pairs64, sc + SC_PAIRS64, 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&ctx->out_h->st_pairs64, sc + SC_STPAIRS64, 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&ctx->out_h->sort_fault, sc + SC_FAULT, 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&ctx->out_h->overflow, sc + SC_OVERFLOW, 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&ctx->out_h->visible, sc + SC_VISIBLE, 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(ctx->out_h->losses, losses_dev, sizeof(float) * V, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(ctx->out_h, ctx->scalars.p, sizeof(StepOut), cudaMemcpyDeviceToHost, st);
     }
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
@@ -1563,12 +1574,10 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
         // budget, go to the groups directly instead of through a full attempt
         // that would overflow its pair buffer.
         const DevCam* cams_dev = (const DevCam*)((char*)ctx->hdr.p + offsetof(StepHdr, cams));
-        uint32_t* sc = ctx->scalars.as<uint32_t>();
         CK(cudaMemcpyAsync(ctx->hdr.p, ctx->hdr_h, sizeof(StepHdr), cudaMemcpyHostToDevice, ctx->st));
-        CK(cudaMemsetAsync(sc + SC_VISIBLE, 0, 4, ctx->st));
         launch_project(s.params.as<float4>(), s.n, s.cap, cams_dev, V, ctx->opt.tile_w, ctx->opt.tile_h, ctx->rec.as<float4>(),
-                       ctx->cnt.as<uint32_t>(), ctx->tdesc.as<uint2>(), ctx->dkey.as<uint32_t>(), ctx->ids.as<uint32_t>(),
-                       zero_bg(bg) ? 1 : 0, sc + SC_VISIBLE, ctx->gcache.as<float4>(), ctx->spans.as<uint4>(), ctx->st);
+                       ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), zero_bg(bg) ? 1 : 0, ctx->gcache.as<float4>(),
+                       ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), ctx->st);
         launch_view_pairs(ctx->cnt.as<uint32_t>(), (uint32_t)s.n, V, ctx->view_pairs.as<unsigned long long>(), ctx->st);
         CK(cudaGetLastError());
         unsigned long long per[MAX_VIEWS], total = 0;
@@ -1585,13 +1594,11 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
         h->bc[1] = 1.0f - powi_f(tc.beta2, (int)s.t);
         // Everything a captured graph bakes in: sizes, every buffer address, and
         // the loss weight, background and optimiser constants.
-        const DBuf* bufs[] = {&s.params, &s.grads, &s.m1, &s.m2, &s.accum, &s.denom, &ctx->rec, &ctx->cnt, &ctx->tdesc, &ctx->spans, &ctx->gv, &ctx->gcache, &ctx->dkey,
-                              &ctx->ids, &ctx->ckey, &ctx->cslot, &ctx->chunk_counts, &ctx->st_cnt, &ctx->st_desc,
-                              &ctx->st_masks, &ctx->st_chunks, &ctx->st_planes, &ctx->st_block_sums,
-                              &ctx->acc, &ctx->pkeys,
-                              &ctx->pvals, &ctx->ranges, &ctx->rgb, &ctx->final_t,
-                              &ctx->last, &ctx->dl, &ctx->partials, &ctx->scalars, &ctx->block_sums, &ctx->hdr, &ctx->outd,
-                              &ctx->sort.hist, &ctx->sort.keys2, &ctx->sort.vals2};
+        const DBuf* bufs[] = {&s.params, &s.grads, &s.m1, &s.m2, &s.accum, &s.denom, &ctx->rec, &ctx->cnt, &ctx->spans,
+                              &ctx->gv, &ctx->gcache, &ctx->dkey, &ctx->ckey, &ctx->cslot, &ctx->chunk_counts,
+                              &ctx->st_cnt, &ctx->st_masks, &ctx->st_chunks, &ctx->st_planes, &ctx->st_block_sums, &ctx->acc, &ctx->pkeys,
+                              &ctx->pvals, &ctx->ranges, &ctx->rgb, &ctx->final_t, &ctx->last, &ctx->dl, &ctx->partials,
+                              &ctx->scalars, &ctx->hdr, &ctx->sort.hist, &ctx->sort.keys2, &ctx->sort.vals2};
         float fk[14] = {bg[0], bg[1], bg[2], lambda, tc.lr_position, tc.lr_rotation, tc.lr_scale, tc.lr_opacity,
                         tc.lr_sh_dc, tc.lr_sh_rest, tc.beta1, tc.beta2, tc.eps, (float)ctx->opt.reference_compat};
         auto make_key = [&]() {
@@ -1600,7 +1607,8 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
                                          (uint64_t)(uintptr_t)ctx->st, (uint64_t)ctx->opt.tile_w,
                                          (uint64_t)ctx->opt.tile_h, (uint64_t)ctx->opt.batch,
                                          (uint64_t)ctx->opt.pixels_per_thread, (uint64_t)(host_targets != nullptr),
-                                         (uint64_t)accumulate};
+                                         (uint64_t)accumulate, (uint64_t)supertile_cap(ctx, V),
+                                         (uint64_t)ctx->wide_supertiles};
             for (const DBuf* b : bufs) key.push_back((uint64_t)(uintptr_t)b->p);
             for (float f : fk) {
                 uint32_t u;
@@ -1631,14 +1639,14 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
             for (int i = 0; i <= RGS_NUM_STAGES; ++i) ctx->ev_marked[i] = ctx->graph_marked[i];
             prof_collect(ctx);
         }
-        if (ctx->out_h->sort_fault) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
-        ctx->stats.pairs = ctx->out_h->pairs64;
-        ctx->stats.supertile_entries = ctx->out_h->st_pairs64;
-        ctx->stats.visible = ctx->out_h->visible;
+        if (ctx->out_h->w[SC_FAULT]) return fail(ctx, RGS_ERR_CUDA, "a sort pass's staged copies timed out");
+        ctx->stats.pairs = ctx->out_h->u64(SC_PAIRS64);
+        ctx->stats.supertile_entries = ctx->out_h->u64(SC_STPAIRS64);
+        ctx->stats.visible = ctx->out_h->w[SC_NVIS];
         ctx->stats.view_groups = 1;
-        if (!ctx->out_h->overflow) {
+        if (!ctx->out_h->w[SC_OVERFLOW]) {
             if (losses)
-                for (int v = 0; v < V; ++v) losses[v] = ctx->out_h->losses[v];
+                for (int v = 0; v < V; ++v) losses[v] = ctx->out_h->loss(v);
             if (fused) s.mlen = std::max(s.mlen, s.n);
             ctx->batch_views = allow_split ? V : 0;
             return RGS_OK;
@@ -1648,10 +1656,10 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
         s.t -= tstep;
         ctx->stats.overflow_retries += 1;
         if (accumulate) return fail(ctx, RGS_ERR_CAPACITY, "a view group outgrew its pair buffer");
-        const unsigned long long K = ctx->out_h->pairs64;
+        const unsigned long long K = ctx->out_h->u64(SC_PAIRS64);
         if (K > ctx->opt.batch_pair_limit && allow_split && V > 1) return split_step(ctx, views, V, bg, lambda, tc, losses, fused, host_targets);
         // the supertile entries share the pair buffers: room for both
-        if ((rc = ensure_pairs(ctx, std::max(K, (unsigned long long)ctx->out_h->st_pairs64)))) return rc;
+        if ((rc = ensure_pairs(ctx, std::max(K, ctx->out_h->u64(SC_STPAIRS64))))) return rc;
     }
     return fail(ctx, RGS_ERR_CAPACITY, "pair buffer overflow persisted");
 }
@@ -2176,9 +2184,7 @@ int debug_tile_lists(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_c
     Binned b;
     size_t px, tiles, lb;
     if ((rc = debug_bin(ctx, gaussians, n, camera, dc, &cams_dev, b, px, tiles, lb, prune))) return rc;
-    uint32_t K = 0;
-    CK(cudaMemcpyAsync(&K, ctx->scalars.as<uint32_t>() + SC_PAIRS, 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
+    const uint32_t K = (uint32_t)std::min<unsigned long long>(ctx->out_h->u64(SC_PAIRS64), 0xffffffffull);
     *n_pairs = K;
     if (!entries) return RGS_OK;
     if (!offsets || cap < K) return fail(ctx, RGS_ERR_CAPACITY, "entries buffer too small");
@@ -2210,6 +2216,12 @@ int rgs_debug_tile_lists(rgs_ctx* ctx, const float* gaussians, size_t n, const r
 int rgs_debug_pruned_tile_lists(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera* camera,
                                 uint64_t* n_pairs, int32_t* offsets, int32_t* entries, size_t cap) {
     return debug_tile_lists(ctx, gaussians, n, camera, n_pairs, offsets, entries, cap, true);
+}
+
+int rgs_debug_wide_supertiles(rgs_ctx* ctx, int on) {
+    if (!ctx) return RGS_ERR_INVALID_ARG;
+    ctx->wide_supertiles = on != 0;
+    return RGS_OK;
 }
 
 int rgs_debug_forward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera* camera, const float bg[3], float* rgb,
@@ -2246,7 +2258,7 @@ int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs
     if ((rc = upload_single_cam(ctx, dc, &cams_dev))) return rc;
     BlendArgs fa = blend_args(ctx, ctx->sc, cams_dev, 1, nullptr, tiles, b, bg, true);
     launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
-    float* losses_dev = (float*)((char*)ctx->outd.p + offsetof(StepOut, losses));
+    float* losses_dev = losses_of(ctx);
     CK(launch_loss(cams_dev, 1, (int)lb, ctx->rgb.as<float>(), lambda, ctx->dl.as<float>(), ctx->partials.as<float>(),
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, ctx->st));
     CK(cudaMemsetAsync(ctx->acc.p, 0, std::max<size_t>(n, 1) * 3 * sizeof(float4), ctx->st));

@@ -161,20 +161,25 @@ void launch_aos_to_grad_planes(const float* aos, float4* planes, int n, int cap,
 void launch_check_finite(const float4* planes, int n, int cap, int* flag, cudaStream_t st);
 
 // project.cu
-// tdesc[s] = (global id of the splat's first CTA tile, width | height << 16 of
-// its CTA-tile rectangle), cnt[s] = its number of CTA tiles, or with prune = 1
-// the number inside the rows' kept spans (tiles.cuh); zero for culled slots.
-// *visible (zeroed by the caller) gains the number of slots with cnt > 0.
-// With prune, spans[2 slot] holds the kept spans of rectangles up to SPAN_ROWS
-// rows and 15 columns, byte r of the 16 (x holds rows 0-3, y 4-7, ...): first
-// kept column - first rectangle column | kept count << 4. Larger rectangles
-// get SPANS_NONE in every word (a byte 0xff never occurs in a packed record:
-// the first column and the count add up to at most 15).
+// cnt[s] = number of CTA tiles slot s is binned into: those of its rectangle,
+// or with prune = 1 those inside the rows' kept spans (tiles.cuh); zero for
+// culled slots, of which nothing else is written.
+// spans[2 s], spans[2 s + 1]: the slot's 32-byte bin record.
+//   [0] with prune, the kept spans of rectangles up to SPAN_ROWS rows and 15
+//       columns, byte r of the 16 (x holds rows 0-3, y 4-7, ...): first kept
+//       column - first rectangle column | kept count << 4. Larger rectangles
+//       have SPANS_NONE in every word (a byte 0xff never occurs in a packed
+//       record: the first column and the count add up to at most 15).
+//   [1] (first CTA-tile column | row << 16, rect width | height << 16 in CTA
+//       tiles, supertile entries, 0): the slot is binned into the supertiles its
+//       rectangle meets, or with prune, per supertile row, those from the first
+//       to the last that its kept spans meet.
+// st_cnt[s] = the entries again (their scan gathers four bytes a slot).
 constexpr int SPAN_ROWS = 16;
 constexpr uint32_t SPANS_NONE = 0xffffffffu;
 void launch_project(const float4* params, int n, int cap, const DevCam* cams, int nviews,
-                    int tile_w, int tile_h, float4* rec, uint32_t* cnt, uint2* tdesc, uint32_t* dkey,
-                    uint32_t* ids, int prune, uint32_t* visible, float4* gcache, uint4* spans, cudaStream_t st);
+                    int tile_w, int tile_h, float4* rec, uint32_t* cnt, uint32_t* dkey, int prune, float4* gcache,
+                    uint4* spans, uint32_t* st_cnt, cudaStream_t st);
 // Per-Gaussian view-independent projection terms ([2][cap] float4: opacity
 // and the 3D covariance's six entries), computed by launch_project first and
 // read by the geometry of the same step.
@@ -182,7 +187,7 @@ void launch_gauss_cache(const float4* params, int n, int cap, float4* gcache, cu
 void launch_project_wgsl(const float4* params, int n, int cap, const DevCam* cam, int cpu_math,
                          float* splats10, uint32_t* keys, cudaStream_t st);
 void launch_composite_prepare(const float* splats10, int n, const DevCam* cam, int tile_w, int tile_h,
-                              float4* rec, uint32_t* cnt, uint2* tdesc, uint32_t* dkey, uint32_t* ids,
+                              float4* rec, uint32_t* cnt, uint32_t* dkey, uint4* spans, uint32_t* st_cnt,
                               cudaStream_t st);
 
 // sort.cu: stable LSD radix sort of (key, value) u32 pairs on bits [0, bits).
@@ -195,45 +200,58 @@ int sort_grid_blocks();
 inline size_t sort_hist_bytes(int grid) { return ((size_t)grid * 256 + 256) * 4; }
 
 // bin.cu
-// Exclusive scan of the per-slot counts cnt[order[r]] in depth order (pruned
-// tile pairs, or supertile entries). block_sums: one u64 per CTA of `grid`;
-// *total is the count saturated at 2^32 - 1, *total64 the exact count.
-// S_dev (may be null) holds the number of order entries on the device.
-void launch_count_scan(const uint32_t* order, const uint32_t* cnt, uint32_t S, const uint32_t* S_dev,
-                       unsigned long long* block_sums, uint32_t* total, unsigned long long* total64, int grid, cudaStream_t st);
 // Per-view pair totals (slot = view * n + Gaussian) into out[0, V).
 void launch_view_pairs(const uint32_t* cnt, uint32_t n, int V, unsigned long long* out, cudaStream_t st);
-int bin_grid_blocks();
+int bin_grid_blocks(size_t S);
+int bin_grid_max();
 // The slots with at least one tile pair (cnt != 0), gathered in slot order:
 // their keys into ckey, their slot indices into cslot, the count into *n_out
-// (and *n_out64). chunk_counts holds compact_chunks(S) u64.
+// (and *n_out64); *pairs64 (zeroed by the caller) gains the sum of cnt.
+// chunk_counts holds compact_chunks(S) u64.
 size_t compact_chunks(size_t S);
 void launch_compact_visible(const uint32_t* cnt, const uint32_t* key, uint32_t S, unsigned long long* chunk_counts,
                             uint32_t* ckey, uint32_t* cslot, uint32_t* n_out, unsigned long long* n_out64,
-                            const uint2* tdesc, const DevCam* cams, uint32_t n_per_view, uint32_t* st_cnt, uint2* st_desc,
-                            cudaStream_t st);
-// Supertile rectangles expanded into (supertile id, slot) entries in the
-// order's (depth) order: the rectangle emitter with the view's supertile
-// stride (st_desc holds the first supertile id and width | height << 16).
-void launch_emit_supertiles(const uint32_t* order, const uint2* st_desc, uint32_t S, const uint32_t* S_dev,
-                            const unsigned long long* block_sums, uint32_t* keys, uint32_t* vals, uint32_t cap, int* overflow,
-                            const uint32_t* total, uint32_t* eff, const DevCam* cams, uint32_t n_per_view, int grid,
-                            cudaStream_t st);
+                            unsigned long long* pairs64, cudaStream_t st);
+// The depth-ordered slots expanded into (supertile id, slot) entries. First an
+// exclusive scan of their entry counts over the blocks of the emitting grid, in
+// 64 bits (block_sums: one u64 per block; *total is the count saturated at
+// 2^32 - 1, *total64 the exact one), then the emission. With packed, an entry's
+// key holds its 16-tile mask in the upper half (supertile ids then fit 16 bits).
+struct EmitArgs {
+    const uint32_t* order;
+    const uint32_t* n_order;       // device count of the order
+    const uint4* spans;            // bin records (launch_project)
+    const uint32_t* st_cnt;        // supertile entries per slot (the records' third word, apart)
+    const float4* rec;             // splat records (three planes of S)
+    uint32_t S;
+    const DevCam* cams;
+    uint32_t n_per_view;
+    int tile_w, tile_h, prune, packed;
+    unsigned long long* block_sums;
+    uint32_t* total;
+    unsigned long long* total64;
+    uint32_t* keys;
+    uint32_t* vals;
+    uint32_t cap;
+    uint32_t* eff;                 // entries held: min(total, cap)
+    int* overflow;
+};
+void launch_entry_scan(const EmitArgs& a, int grid, cudaStream_t st);
+void launch_emit_supertiles(const EmitArgs& a, int grid, cudaStream_t st);
 
 // supertile.cu: the tile lists from the supertile-sorted entries.
 struct SupertileArgs {
     const DevCam* cams;
     int nviews;
-    const uint32_t* ent_key;       // sorted entries: supertile id
+    const uint32_t* ent_key;       // sorted entries: supertile id (with packed: | tile mask << 16)
     const uint32_t* ent_slot;      // sorted entries: slot
     const uint32_t* n_ent;         // device count of the sorted entries
-    const uint2* tdesc;            // per slot: first CTA tile, rect width | height << 16
-    const uint4* spans;            // per slot (with prune), 32 B: packed kept spans (or SPANS_NONE), then tdesc
+    const uint4* spans;            // bin records (launch_project)
     const float4* rec;             // splat records (three planes of S)
     uint32_t S;
     uint32_t n_per_view;           // slot = view * n_per_view + Gaussian
-    int tile_w, tile_h, prune;
-    uint16_t* masks;               // per entry: the supertile's tiles it keeps (bit = row * 4 + col)
+    int tile_w, tile_h, prune, packed;
+    uint16_t* masks;               // not packed: per entry the supertile's tiles it keeps (bit = row * 4 + col)
     uint32_t* chunk_cnt;           // [tile position][chunk_stride] entries per chunk, scanned in place
     uint32_t chunk_stride;         // supertile_chunks(cap)
     uint32_t* plane_tot;           // [tile position] entries with that bit
@@ -264,7 +282,7 @@ struct BlendArgs {
     int* last;
     const float* dl;
     float4* acc;
-    uint32_t* work;                // dynamic tile counter (zeroed by the launcher)
+    uint32_t* work;                // dynamic tile counter (zeroed by the binning before it)
     int rect_filter;               // per-pixel reference-tile membership test
     int empty_tile_black;          // pixels of empty reference tiles render 0, not bg
     int pixels_per_thread;         // 1: two pixels per thread; 2: four, or two where tiles are few

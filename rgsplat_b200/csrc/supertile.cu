@@ -7,14 +7,15 @@
 // sort of (supertile, slot) entries. The sorted entries are then cut into
 // chunks of ST_CHUNK, whatever supertiles they belong to, so every CTA gets
 // the same work however unevenly the splats crowd the supertiles:
-//   k_st_masks: per entry, the tiles of its supertile the slot keeps (the
-//               rectangle, or with pruning each tile row's kept span, read
-//               from the spans the projection packed in the slot's 32-byte
-//               record, or for rectangles too large to pack recomputed by
-//               the same test on the same floats the projection counted
-//               with) as a 16-bit mask, bit t for tile position
-//               t = row * ST_EDGE + col; per chunk and position, the entries
-//               with that bit set (packed byte counters);
+//   k_st_counts: per chunk and tile position, the entries whose 16-bit mask of
+//               the supertile's tiles the slot keeps has that bit (bit t for
+//               tile position t = row * ST_EDGE + col). The mask comes with the
+//               entry, in the upper half of its sort key;
+//   k_st_masks: the same for batches whose supertile ids need more than 16
+//               bits: the masks are formed here, from the slot's bin record (the
+//               rectangle, or with pruning each tile row's kept span, packed
+//               there or for large rectangles recomputed by the same test on
+//               the same floats the projection counted with);
 //   k_st_scan:  one CTA per position: an exclusive scan of its chunk counts;
 //   k_st_lists: the lists. The pairs of position t form plane t of the list
 //               buffer, in entry order, the planes one after another; the
@@ -52,22 +53,13 @@ struct SlotRect {
     int cx0, ty0, w, h;
 };
 
-__device__ __forceinline__ SlotRect slot_rect(const DevCam& c, uint2 d) {
+__device__ __forceinline__ SlotRect slot_rect(uint2 d) {
     SlotRect q;
-    const int lt = (int)d.x - c.tile_base;
-    q.ty0 = lt / c.tiles_x;
-    q.cx0 = lt - q.ty0 * c.tiles_x;
+    q.cx0 = (int)(d.x & 0xffffu);
+    q.ty0 = (int)(d.x >> 16);
     q.w = (int)(d.y & 0xffffu);
     q.h = (int)(d.y >> 16);
     return q;
-}
-
-// Bits of row k of a supertile whose first column is q0 for the kept columns
-// [c0, c1): bit k * ST_EDGE + q for column q0 + q.
-__device__ __forceinline__ uint32_t row_bits(int c0, int c1, int q0, int k) {
-    c0 = max(c0, q0);
-    c1 = min(c1, q0 + ST_EDGE);
-    return c1 > c0 ? ((1u << (c1 - c0)) - 1u) << (k * ST_EDGE + (c0 - q0)) : 0u;
 }
 
 // The tiles of supertile (sx, sy) the slot's rectangle holds (no pruning).
@@ -146,7 +138,6 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_st_masks(SupertileArgs a) {
     __shared__ uint32_t s_w[ST_WARPS][4];
     const uint32_t* __restrict__ ent_key = a.ent_key;
     const uint32_t* __restrict__ ent_slot = a.ent_slot;
-    const uint2* __restrict__ tdesc = a.tdesc;
     const uint4* __restrict__ spans = a.spans;
     const uint32_t n = st_entries(a), nch = (n + ST_CHUNK - 1) / ST_CHUNK;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -167,14 +158,10 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_st_masks(SupertileArgs a) {
             sp[r] = make_uint4(0u, 0u, 0u, 0u);
             d[r] = make_uint2(0u, 0u);
             if (e < n) {
-                if (a.prune) {
-                    // one 32-byte record: the spans, then the rectangle
-                    sp[r] = spans[2 * (size_t)slot[r]];
-                    const uint4 td = spans[2 * (size_t)slot[r] + 1];
-                    d[r] = make_uint2(td.x, td.y);
-                } else {
-                    d[r] = tdesc[slot[r]];
-                }
+                // one 32-byte record: the spans, then the rectangle
+                if (a.prune) sp[r] = spans[2 * (size_t)slot[r]];
+                const uint4 td = spans[2 * (size_t)slot[r] + 1];
+                d[r] = make_uint2(td.x, td.y);
             }
         }
         uint32_t acc[4] = {0u, 0u, 0u, 0u};
@@ -184,7 +171,7 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_st_masks(SupertileArgs a) {
             if (e < n) {
                 const DevCam& c = a.cams[slot[r] / a.n_per_view];
                 const int local = (int)st[r] - c.st_base, sy = local / c.st_x, sx = local - sy * c.st_x;
-                const SlotRect q = slot_rect(c, d[r]);
+                const SlotRect q = slot_rect(d[r]);
                 const uint32_t m = !a.prune                                 ? mask_rect(q, sx, sy)
                                    : (sp[r].x & 0xffu) != (SPANS_NONE & 0xffu) ? mask_packed(q, sp[r], sx, sy)
                                                       : mask_computed(a.rec, a.S, a.tile_w, a.tile_h, c.height, slot[r], q,
@@ -195,6 +182,35 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_st_masks(SupertileArgs a) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) acc[k] += x[k];
             }
+        }
+        warp_counts(acc, lane, s_w[w]);
+        __syncthreads();
+        if (threadIdx.x < ST_TILES) {
+            const int t = threadIdx.x;
+            uint32_t s = 0;
+#pragma unroll
+            for (int k = 0; k < ST_WARPS; ++k) s += byte_of(s_w[k][t >> 2], t & 3);
+            a.chunk_cnt[(size_t)t * a.chunk_stride + ch] = s;
+        }
+        __syncthreads();
+    }
+}
+
+// The chunk counts alone, from masks that came with the sorted keys.
+__global__ void __launch_bounds__(ST_THREADS) k_st_counts(SupertileArgs a) {
+    __shared__ uint32_t s_w[ST_WARPS][4];
+    const uint32_t* __restrict__ ent_key = a.ent_key;
+    const uint32_t n = st_entries(a), nch = (n + ST_CHUNK - 1) / ST_CHUNK;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (uint32_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+        uint32_t acc[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int r = 0; r < ST_RUN; ++r) {
+            const uint32_t e = ch * ST_CHUNK + threadIdx.x + (uint32_t)(ST_THREADS * r);
+            uint32_t x[4];
+            spread_mask(e < n ? ent_key[e] >> 16 : 0u, x);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] += x[k];
         }
         warp_counts(acc, lane, s_w[w]);
         __syncthreads();
@@ -257,6 +273,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_st_scan(SupertileArgs a) {
 // entry's place in plane t: the warp's start in that plane (s_base) + the
 // entries of the warp's earlier rounds and earlier lanes with bit t, read off
 // a lane scan of the byte counters.
+template <bool PACKED>
 __global__ void __launch_bounds__(ST_THREADS) k_st_lists(SupertileArgs a) {
     __shared__ uint32_t s_w[ST_WARPS][4];
     // the warp's start in each plane, clamped to the capacity: every place
@@ -267,6 +284,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_st_lists(SupertileArgs a) {
     const uint32_t* __restrict__ ent_slot = a.ent_slot;
     const uint16_t* __restrict__ masks = a.masks;
     const uint32_t n = st_entries(a), nch = (n + ST_CHUNK - 1) / ST_CHUNK;
+    const uint32_t id_bits = PACKED ? 0xffffu : 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // lane t: where plane t starts (the planes before it, in 64 bits)
     unsigned long long plane0 = 0;
@@ -279,8 +297,9 @@ __global__ void __launch_bounds__(ST_THREADS) k_st_lists(SupertileArgs a) {
         for (int r = 0; r < ST_RUN; ++r) {
             const uint32_t e = e0 + (uint32_t)(32 * r);
             const bool valid = e < n;
-            m[r] = valid ? (uint32_t)masks[e] : 0u;
-            key[r] = valid ? ent_key[e] : 0xffffffffu;
+            const uint32_t kv = valid ? ent_key[e] : 0u;
+            m[r] = PACKED ? kv >> 16 : valid ? (uint32_t)masks[e] : 0u;
+            key[r] = !valid ? 0xffffffffu : PACKED ? kv & 0xffffu : kv;
             slot[r] = valid ? ent_slot[e] : 0u;
             uint32_t x[4];
             spread_mask(m[r], x);
@@ -335,8 +354,8 @@ __global__ void __launch_bounds__(ST_THREADS) k_st_lists(SupertileArgs a) {
             uint32_t next = __shfl_down_sync(0xffffffffu, key[r], 1);
             const uint32_t pw = r > 0 ? __shfl_sync(0xffffffffu, key[r > 0 ? r - 1 : 0], 31) : 0u;
             const uint32_t nw = r + 1 < ST_RUN ? __shfl_sync(0xffffffffu, key[r + 1 < ST_RUN ? r + 1 : r], 0) : 0u;
-            if (lane == 0) prev = r > 0 ? pw : (valid && e > 0 ? ent_key[e - 1] : 0xffffffffu);
-            if (lane == 31) next = r + 1 < ST_RUN ? nw : (valid && e + 1 < n ? ent_key[e + 1] : 0xffffffffu);
+            if (lane == 0) prev = r > 0 ? pw : (valid && e > 0 ? ent_key[e - 1] & id_bits : 0xffffffffu);
+            if (lane == 31) next = r + 1 < ST_RUN ? nw : (valid && e + 1 < n ? ent_key[e + 1] & id_bits : 0xffffffffu);
             const bool first = valid && prev != key[r], last = valid && next != key[r];
             if (first || last) {
                 // a supertile's first entry starts, its last ends, the lists
@@ -362,9 +381,11 @@ __global__ void __launch_bounds__(ST_THREADS) k_st_lists(SupertileArgs a) {
 
 void launch_supertile_lists(const SupertileArgs& a, cudaStream_t st) {
     const int grid = (int)std::max<size_t>(1, std::min<size_t>(a.chunk_stride, (size_t)device_sm_count() * 8));
-    k_st_masks<<<grid, ST_THREADS, 0, st>>>(a);
+    if (a.packed) k_st_counts<<<grid, ST_THREADS, 0, st>>>(a);
+    else k_st_masks<<<grid, ST_THREADS, 0, st>>>(a);
     k_st_scan<<<ST_TILES, SCAN_THREADS, 0, st>>>(a);
-    k_st_lists<<<grid, ST_THREADS, 0, st>>>(a);
+    if (a.packed) k_st_lists<true><<<grid, ST_THREADS, 0, st>>>(a);
+    else k_st_lists<false><<<grid, ST_THREADS, 0, st>>>(a);
 }
 
 }  // namespace rgs

@@ -71,7 +71,14 @@ __device__ __forceinline__ void cta_tile_box(int tx, int ty, int tw, int th, int
 // for xl (the roots are formed with 1/a, within an ulp of the quotient). The
 // span is computed with T enlarged by 2 % and widened by half a pixel, so it
 // contains every tile the per-tile test keeps with a margin far above float
-// rounding; the blend still applies the per-tile test.
+// rounding (and above that of the approximate square roots and quotients used
+// here); the blend still applies its own tests.
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 struct SpanSetup {
     float sx, sy, a, b, c, T, xr, yr, ia;  // ia = 1 / a
     bool testable;
@@ -83,9 +90,9 @@ __device__ __forceinline__ SpanSetup span_setup(float sx, float sy, float a, flo
     u.testable = a > 0.0f && c > 0.0f && (a * c - b * b) >= 0.01f * (a * c);
     u.T = -2.0f * thr / 0.999f * 1.02f;
     const float det = a * c - b * b;
-    u.xr = u.testable ? sqrtf(u.T * c / det) : 0.0f;
-    u.yr = u.testable ? -b / c * u.xr : 0.0f;
-    u.ia = u.testable ? 1.0f / a : 0.0f;
+    u.xr = u.testable ? sqrt_approx(__fdividef(u.T * c, det)) : 0.0f;
+    u.yr = u.testable ? __fdividef(-b, c) * u.xr : 0.0f;
+    u.ia = u.testable ? __fdividef(1.0f, a) : 0.0f;
     return u;
 }
 
@@ -107,7 +114,7 @@ __device__ __forceinline__ void kept_cols(const SpanSetup& u, int ty, int tw, in
             c1 = c0;
             return;
         }
-        xr = (-u.b * er + sqrtf(disc)) * u.ia;
+        xr = (-u.b * er + sqrt_approx(disc)) * u.ia;
     }
     const float el = fminf(fmaxf(-u.yr, ly), hy);
     if (el == -u.yr) {
@@ -118,7 +125,7 @@ __device__ __forceinline__ void kept_cols(const SpanSetup& u, int ty, int tw, in
             c1 = c0;
             return;
         }
-        xl = (-u.b * el - sqrtf(disc)) * u.ia;
+        xl = (-u.b * el - sqrt_approx(disc)) * u.ia;
     }
     // pixel-space interval, widened by half a pixel; a tile's pixel centres
     // span [tx * tw + 0.5, tx * tw + tw - 0.5]
@@ -130,6 +137,14 @@ __device__ __forceinline__ void kept_cols(const SpanSetup& u, int ty, int tw, in
     c0 = (int)fminf(fmaxf(f0, (float)cx0), (float)cx1);
     c1 = (int)fminf(fmaxf(f1, (float)cx0), (float)cx1);
     if (c1 < c0) c1 = c0;
+}
+
+// Bits of row k of a supertile whose first column is q0 for the kept columns
+// [c0, c1): bit k * ST_EDGE + q for column q0 + q.
+__device__ __forceinline__ uint32_t row_bits(int c0, int c1, int q0, int k) {
+    c0 = max(c0, q0);
+    c1 = min(c1, q0 + ST_EDGE);
+    return c1 > c0 ? ((1u << (c1 - c0)) - 1u) << (k * ST_EDGE + (c0 - q0)) : 0u;
 }
 
 }  // namespace rgs
