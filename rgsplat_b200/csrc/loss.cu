@@ -9,18 +9,16 @@
 //
 // B200 mapping: one CTA per 32x32 output tile of any view of the batch. The
 // CTA stages the rendered and target channels over a 52x52 region (two
-// 5-pixel halos) in shared memory and runs all ten blurs there, so HBM sees
+// 5-pixel halos) in shared memory and runs all blurs there, so HBM sees
 // each input pixel about once and dL/dpixel is written once. The blurs are
 // register-blocked (a thread produces a run of outputs from one sliding
-// window, so each shared-memory value and each product x^2, y^2, xy is
-// formed once per run). Two kernels: k_loss keeps the reference's separate
-// multiply and add per tap and its divisions (dL/dpixel bit-identical,
-// rgs_options.exact_loss); k_loss_fused, the default, accumulates with fused
-// multiply-adds on packed f32x2 pairs and forms the three SSIM quotients from
-// one reciprocal. The scalar loss is reduced per CTA and then per view in a
-// fixed order (deterministic). (Staging each channel by 4-byte asynchronous
-// copies issued during the previous channel's passes 2-4, with the tile's
-// centre kept apart for pass 4, measured slower: 0.84 against 0.80 ms.)
+// window, so each shared-memory value and each product is formed once per run).
+// Two kernels: k_loss keeps the reference's separate multiply and add per tap and
+// its divisions (dL/dpixel bit-identical, rgs_options.exact_loss); k_loss_fused,
+// the default, accumulates with fused multiply-adds on packed f32x2 pairs and
+// forms the SSIM quotients from one reciprocal. The scalar loss is reduced per
+// CTA and then per view in a fixed order (deterministic).
+#include <algorithm>
 #include <mutex>
 
 #include "rgs_internal.cuh"
@@ -285,33 +283,80 @@ __global__ void __launch_bounds__(LOSS_THREADS) k_loss(const DevCam* __restrict_
 }
 
 // The same loss with fused multiply-adds, two independent accumulators per
-// packed f32x2 instruction (per lane the same rounding as one fmaf): the
-// statistics as (x, y), (x^2, y^2), xy; the maps as (P, Q), (R, Q mu_y),
-// R mu_x. Pass outputs live in shared memory as float2 planes of those pairs
-// (plus one float plane), in the same regions as the exact kernel's.
+// packed f32x2 instruction (per lane the rounding of one fmaf): the statistics
+// as (x, y), (x^2, y^2), xy; the maps as (P, Q), (R, Q mu_y), R mu_x. Pass
+// outputs live in shared memory as float2 planes of those pairs (plus one float
+// plane).
+//
+// What bounds it: FMA issue (339 fused multiply-adds per pixel and channel with
+// the halos) and the latency around the four barriers per channel. Ten warps
+// share a 32x32 tile: with runs of 7, 6, 8 and 4 outputs the four passes have
+// 312, 294, 168 and 256 work items for 320 threads (256 threads leave the first
+// pass a second round that is three quarters empty). The maps reuse the input's
+// shared memory and pass 3's output that of pass 1; the tile arrives a row per
+// warp by 4-byte asynchronous copies, the next channel's while this one's last
+// pass runs; rows are padded against bank conflicts. 0.84 -> 0.77 ms (1M
+// Gaussians x 8 views, 8.5M pixels), 162 -> 151 us (1600x1064), 20.0 -> 17.5 us
+// (256x256). 256 and 384 threads 0.85 and 0.83 ms.
+//
+// Fewer blurs would do: P', (Q mu_y)' and (R mu_x)' enter the gradient as one
+// sum, and E[x^2] + E[y^2] as one; seven blurs ran 0.60 ms, eight 0.71. Not
+// kept: the variances and the gradient's terms cancel to 1e-3 of their size, so
+// either form carries a rounding error of 2 to 4e-5 of the gradient's norm, and
+// two forms differ by as much from one another.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-__global__ void __launch_bounds__(LOSS_THREADS) k_loss_fused(const DevCam* __restrict__ cams, int nviews,
-                                                             const uint32_t* total_dev, int total_host,
-                                                             const float* __restrict__ rgb, float lambda,
-                                                             float* __restrict__ dl, float* __restrict__ partials) {
-    extern __shared__ float smem[];
-    float* in_x = smem;
-    float* in_y = in_x + RG * RG;
-    float* tmp = in_y + RG * RG;   // pass 1 out: float2 [RG][MG] x2 + float [RG][MG]; pass 3 out: [MG][LTP] likewise
-    float* st = tmp + 5 * RG * MG;  // pass 2 out (maps): float2 [MG][MGP] x2 + float [MG][MGP]
-    float* kw = st + 5 * MG * MGP;
+constexpr int FL_THREADS = 320;
+constexpr int FL_WARPS = FL_THREADS / 32;
+constexpr int FH1 = 7, FV1 = 6, FH2 = 8, FV2 = 4;  // run lengths of the four passes
+constexpr int FRS = RG + 1;   // row strides (float2 / float)
+constexpr int FTS = MG + 1;
+constexpr int FGS = LT + 1;
+static_assert(MG % FH1 == 0 && MG % FV1 == 0 && LT % FH2 == 0 && LT % FV2 == 0, "run lengths must tile the regions");
+constexpr size_t FL_IN = sizeof(float2) * RG * FRS;                                   // x, y
+constexpr size_t FL_MAPS = (2 * sizeof(float2) + sizeof(float)) * MG * FTS;            // (P, Q), (R, Q mu_y), R mu_x
+constexpr size_t FL_AREA0 = ((FL_IN > FL_MAPS ? FL_IN : FL_MAPS) + 15) & ~(size_t)15;
+constexpr size_t FL_AREA1 = (2 * sizeof(float2) + sizeof(float)) * RG * FTS;          // pass 1 out; then pass 3 out
+constexpr size_t FL_SMEM = FL_AREA0 + FL_AREA1 + sizeof(float) * (16 + 2 * FL_WARPS);
+static_assert(FL_AREA0 % 16 == 0 && FL_AREA1 % 16 == 0, "each area starts on a float2 boundary");
+static_assert((2 * sizeof(float2) + sizeof(float)) * MG * FGS <= FL_AREA1, "pass-3 output must fit in the pass-1 buffer");
+
+// Four bytes global -> shared, asynchronously; zero when !in (nothing is read).
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(in ? 4 : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ float fl_block_sum(float v, float* s_red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float t = 0.0f;
+    for (int k = 0; k < FL_WARPS; ++k) t += s_red[k];
+    return t;
+}
+
+__global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __restrict__ cams, int nviews,
+                                                              const uint32_t* total_dev, int total_host,
+                                                              const float* __restrict__ rgb, float lambda,
+                                                              float* __restrict__ dl, float* __restrict__ partials) {
+    extern __shared__ __align__(16) unsigned char fl_smem[];
+    float2* in = reinterpret_cast<float2*>(fl_smem);               // [RG][FRS]
+    float2* m01 = reinterpret_cast<float2*>(fl_smem);              // [MG][FTS], over the input
+    float2* m23 = m01 + MG * FTS;
+    float* m4 = reinterpret_cast<float*>(m23 + MG * FTS);
+    float2* t01 = reinterpret_cast<float2*>(fl_smem + FL_AREA0);   // [RG][FTS]: mu_x, mu_y
+    float2* t23 = t01 + RG * FTS;                                  // E[x^2], E[y^2]
+    float* t4 = reinterpret_cast<float*>(t23 + RG * FTS);          // E[xy]
+    float2* g01 = reinterpret_cast<float2*>(fl_smem + FL_AREA0);   // [MG][FGS], over pass 1's output
+    float2* g23 = g01 + MG * FGS;
+    float* g4 = reinterpret_cast<float*>(g23 + MG * FGS);
+    float* kw = reinterpret_cast<float*>(fl_smem + FL_AREA0 + FL_AREA1);
     float* s_red = kw + 16;
-    float2* t01 = reinterpret_cast<float2*>(tmp);
-    float2* t23 = t01 + RG * MG;
-    float* t4 = reinterpret_cast<float*>(t23 + RG * MG);
-    float2* m01 = reinterpret_cast<float2*>(st);
-    float2* m23 = m01 + MG * MGP;
-    float* m4 = reinterpret_cast<float*>(m23 + MG * MGP);
-    float2* g01 = reinterpret_cast<float2*>(tmp);
-    float2* g23 = g01 + MG * LTP;
-    float* g4 = reinterpret_cast<float*>(g23 + MG * LTP);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         // gaussian_kernel_1d(5, 1.5), backward.rs:759-772
         float sum = 0.0f;
@@ -324,9 +369,10 @@ __global__ void __launch_bounds__(LOSS_THREADS) k_loss_fused(const DevCam* __res
         for (int i = 0; i < 11; ++i) kw[i] = v[i] / sum;
     }
     __syncthreads();
-    float2 ww[11];  // the taps, duplicated for the packed lanes
+    float2 ww[6];  // the taps (symmetric), duplicated for the packed lanes
 #pragma unroll
-    for (int k = 0; k < 11; ++k) ww[k] = f2(kw[k], kw[k]);
+    for (int k = 0; k < 6; ++k) ww[k] = f2(kw[k], kw[k]);
+    auto tap = [&](int k) { return ww[k < 6 ? k : 10 - k]; };
     const int total = total_dev ? (int)*total_dev : total_host;
     for (int blk = blockIdx.x; blk < total; blk += gridDim.x) {
         int v = 0;
@@ -336,192 +382,192 @@ __global__ void __launch_bounds__(LOSS_THREADS) k_loss_fused(const DevCam* __res
         const int lb = blk - c.loss_base;
         const int ox = (lb % c.loss_bx) * LT, oy = (lb / c.loss_bx) * LT;
         const float m_total = (float)((size_t)w * h * 3);
+        const float g_l1 = (1.0f - lambda) / m_total;  // times +-1: the reference's quotient exactly
         const float* tgt = c.target;
-        const size_t pb = (size_t)c.pix_base;
+        const float* img = rgb + (size_t)c.pix_base * 3;
+        float* grad_out = dl + (size_t)c.pix_base * 3;
         float l1_local = 0.0f, ssim_local = 0.0f;
-        for (int ch = 0; ch < 3; ++ch) {
-            for (int i = tid; i < RG * RG; i += LOSS_THREADS) {
-                int r = i / RG, cc = i - r * RG;
-                int gx = ox - 2 * LR + cc, gy = oy - 2 * LR + r;
-                float xv = 0.0f, yv = 0.0f;
-                if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                    size_t p = (size_t)gy * w + gx;
-                    xv = rgb[(pb + p) * 3 + ch];
-                    yv = tgt[p * 4 + ch];
+        // one row of the region per warp and step, two columns per lane
+        const int gx0 = ox - 2 * LR + lane, gx1 = gx0 + 32;
+        const bool in0 = gx0 >= 0 && gx0 < w, in1 = lane < RG - 32 && gx1 >= 0 && gx1 < w;
+        const ptrdiff_t first = (ptrdiff_t)(oy - 2 * LR + warp) * w + gx0, step = (ptrdiff_t)w * FL_WARPS;
+        auto load = [&](int ch) {
+            const float* pi = img + first * 3 + ch;
+            const float* pt = tgt + first * 4 + ch;
+            float2* dst = in + warp * FRS + lane;
+#pragma unroll 2
+            for (int gy = oy - 2 * LR + warp; gy < oy - 2 * LR + RG; gy += FL_WARPS, pi += step * 3, pt += step * 4, dst += FL_WARPS * FRS) {
+                const bool row = gy >= 0 && gy < h;
+                copy4(&dst[0].x, row && in0 ? pi : img, row && in0);
+                copy4(&dst[0].y, row && in0 ? pt : tgt, row && in0);
+                if (lane < RG - 32) {
+                    copy4(&dst[32].x, row && in1 ? pi + 32 * 3 : img, row && in1);
+                    copy4(&dst[32].y, row && in1 ? pt + 32 * 4 : tgt, row && in1);
                 }
-                in_x[i] = xv;
-                in_y[i] = yv;
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        load(0);
+#pragma unroll 1
+        for (int ch = 0; ch < 3; ++ch) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
-            // pass 1: horizontal blur of (x, y), (x^2, y^2), xy over rows
-            // [0, RG), map columns [0, MG); a run of H1 outputs per thread
-            for (int it = tid; it < RG * (MG / H1); it += LOSS_THREADS) {
-                const int r = it / (MG / H1), c0 = (it - r * (MG / H1)) * H1;
-                const float* rx = in_x + r * RG + c0;
-                const float* ry = in_y + r * RG + c0;
-                float2 a01[H1], a23[H1];
-                float a4[H1];
+            // pass 1: horizontal blur of (x, y), (x^2, y^2), xy over rows [0, RG)
+            for (int it = tid; it < RG * (MG / FH1); it += FL_THREADS) {
+                const int r = it % RG, c0 = (it / RG) * FH1;
+                const float2* row = in + r * FRS + c0;
+                float2 a01[FH1], a23[FH1];
+                float a4[FH1];
 #pragma unroll
-                for (int o = 0; o < H1; ++o) {
+                for (int o = 0; o < FH1; ++o) {
                     a01[o] = a23[o] = f2(0.0f, 0.0f);
                     a4[o] = 0.0f;
                 }
 #pragma unroll
-                for (int j = 0; j < H1 + 10; ++j) {
-                    const float2 xy = f2(rx[j], ry[j]);
-                    const float2 sq = __fmul2_rn(xy, xy);
+                for (int j = 0; j < FH1 + 10; ++j) {
+                    const float2 xy = row[j];
+                    const float2 sp = __fmul2_rn(xy, xy);
                     const float cr = xy.x * xy.y;
 #pragma unroll
-                    for (int o = 0; o < H1; ++o) {
+                    for (int o = 0; o < FH1; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        a01[o] = __ffma2_rn(ww[k], xy, a01[o]);
-                        a23[o] = __ffma2_rn(ww[k], sq, a23[o]);
-                        a4[o] = __fmaf_rn(ww[k].x, cr, a4[o]);
+                        a01[o] = __ffma2_rn(tap(k), xy, a01[o]);
+                        a23[o] = __ffma2_rn(tap(k), sp, a23[o]);
+                        a4[o] = __fmaf_rn(tap(k).x, cr, a4[o]);
                     }
                 }
 #pragma unroll
-                for (int o = 0; o < H1; ++o) {
-                    const int q = r * MG + c0 + o;
-                    t01[q] = a01[o];
-                    t23[q] = a23[o];
-                    t4[q] = a4[o];
+                for (int o = 0; o < FH1; ++o) {
+                    t01[r * FTS + c0 + o] = a01[o];
+                    t23[r * FTS + c0 + o] = a23[o];
+                    t4[r * FTS + c0 + o] = a4[o];
                 }
             }
             __syncthreads();
-            // pass 2: vertical blur -> statistics, then the per-pixel SSIM
-            // maps (zero outside the image)
-            for (int it = tid; it < MG * (MG / V1); it += LOSS_THREADS) {
-                const int cm = it % MG, r0 = (it / MG) * V1;
-                float2 mu01[V1], mu23[V1];
-                float mu4[V1];
+            // pass 2: vertical blur -> statistics, then the per-pixel maps
+            // (zero outside the image)
+            for (int it = tid; it < MG * (MG / FV1); it += FL_THREADS) {
+                const int cm = it % MG, r0 = (it / MG) * FV1;
+                float2 mu[FV1], sq[FV1];
+                float cr[FV1];
 #pragma unroll
-                for (int o = 0; o < V1; ++o) {
-                    mu01[o] = mu23[o] = f2(0.0f, 0.0f);
-                    mu4[o] = 0.0f;
+                for (int o = 0; o < FV1; ++o) {
+                    mu[o] = sq[o] = f2(0.0f, 0.0f);
+                    cr[o] = 0.0f;
                 }
 #pragma unroll
-                for (int j = 0; j < V1 + 10; ++j) {
-                    const int q = (r0 + j) * MG + cm;
-                    const float2 u01 = t01[q], u23 = t23[q];
-                    const float u4 = t4[q];
+                for (int j = 0; j < FV1 + 10; ++j) {
+                    const float2 u = t01[(r0 + j) * FTS + cm], q = t23[(r0 + j) * FTS + cm];
+                    const float e = t4[(r0 + j) * FTS + cm];
 #pragma unroll
-                    for (int o = 0; o < V1; ++o) {
+                    for (int o = 0; o < FV1; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        mu01[o] = __ffma2_rn(ww[k], u01, mu01[o]);
-                        mu23[o] = __ffma2_rn(ww[k], u23, mu23[o]);
-                        mu4[o] = __fmaf_rn(ww[k].x, u4, mu4[o]);
+                        mu[o] = __ffma2_rn(tap(k), u, mu[o]);
+                        sq[o] = __ffma2_rn(tap(k), q, sq[o]);
+                        cr[o] = __fmaf_rn(tap(k).x, e, cr[o]);
                     }
                 }
                 const int gx = ox - LR + cm;
 #pragma unroll
-                for (int o = 0; o < V1; ++o) {
+                for (int o = 0; o < FV1; ++o) {
                     const int rm = r0 + o, gy = oy - LR + rm;
                     float P = 0.0f, Q = 0.0f, R = 0.0f, QM = 0.0f, RM = 0.0f;
                     if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                        const float s = ssim_maps<true>(mu01[o].x, mu01[o].y, mu23[o].x, mu23[o].y, mu4[o], P, Q, R, QM, RM);
-                        if (rm >= LR && rm < LR + LT && cm >= LR && cm < LR + LT) ssim_local += s;
+                        const float ssim = ssim_maps<true>(mu[o].x, mu[o].y, sq[o].x, sq[o].y, cr[o], P, Q, R, QM, RM);
+                        if (rm >= LR && rm < LR + LT && cm >= LR && cm < LR + LT) ssim_local += ssim;
                     }
-                    const int q = rm * MGP + cm;
-                    m01[q] = f2(P, Q);
-                    m23[q] = f2(R, QM);
-                    m4[q] = RM;
+                    m01[rm * FTS + cm] = f2(P, Q);
+                    m23[rm * FTS + cm] = f2(R, QM);
+                    m4[rm * FTS + cm] = RM;
                 }
             }
             __syncthreads();
-            // pass 3: horizontal blur of the maps: rows [0, MG), output cols [0, LT)
-            for (int it = tid; it < MG * (LT / H2); it += LOSS_THREADS) {
-                const int rm = it % MG, c0 = (it / MG) * H2;
-#pragma unroll 1
-                for (int pl = 0; pl < 2; ++pl) {
-                    const float2* row = (pl ? m23 : m01) + rm * MGP + c0;
-                    float2 a[H2];
+            // pass 3: horizontal blur of the maps: rows [0, MG), output columns [0, LT)
+            for (int it = tid; it < MG * (LT / FH2); it += FL_THREADS) {
+                const int rm = it % MG, c0 = (it / MG) * FH2;
+                float2 a[FH2], d[FH2];
+                float e[FH2];
 #pragma unroll
-                    for (int o = 0; o < H2; ++o) a[o] = f2(0.0f, 0.0f);
-#pragma unroll
-                    for (int j = 0; j < H2 + 10; ++j) {
-                        const float2 t = row[j];
-#pragma unroll
-                        for (int o = 0; o < H2; ++o) {
-                            const int k = j - o;
-                            if (k < 0 || k > 10) continue;
-                            a[o] = __ffma2_rn(ww[k], t, a[o]);
-                        }
-                    }
-                    float2* out = (pl ? g23 : g01) + rm * LTP + c0;
-#pragma unroll
-                    for (int o = 0; o < H2; ++o) out[o] = a[o];
-                }
-                {
-                    const float* row = m4 + rm * MGP + c0;
-                    float a[H2];
-#pragma unroll
-                    for (int o = 0; o < H2; ++o) a[o] = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < H2 + 10; ++j) {
-                        const float t = row[j];
-#pragma unroll
-                        for (int o = 0; o < H2; ++o) {
-                            const int k = j - o;
-                            if (k < 0 || k > 10) continue;
-                            a[o] = __fmaf_rn(ww[k].x, t, a[o]);
-                        }
-                    }
-#pragma unroll
-                    for (int o = 0; o < H2; ++o) g4[rm * LTP + c0 + o] = a[o];
-                }
-            }
-            __syncthreads();
-            // pass 4: vertical blur -> gradient, combined with the L1 term
-            for (int it = tid; it < LT * (LT / V2); it += LOSS_THREADS) {
-                const int co = it % LT, r0 = (it / LT) * V2;
-                float2 b01[V2], b23[V2];
-                float b4[V2];
-#pragma unroll
-                for (int o = 0; o < V2; ++o) {
-                    b01[o] = b23[o] = f2(0.0f, 0.0f);
-                    b4[o] = 0.0f;
+                for (int o = 0; o < FH2; ++o) {
+                    a[o] = d[o] = f2(0.0f, 0.0f);
+                    e[o] = 0.0f;
                 }
 #pragma unroll
-                for (int j = 0; j < V2 + 10; ++j) {
-                    const int q = (r0 + j) * LTP + co;
-                    const float2 u01 = g01[q], u23 = g23[q];
-                    const float u4 = g4[q];
+                for (int j = 0; j < FH2 + 10; ++j) {
+                    const int p = rm * FTS + c0 + j;
+                    const float2 t = m01[p], u = m23[p];
+                    const float q = m4[p];
 #pragma unroll
-                    for (int o = 0; o < V2; ++o) {
+                    for (int o = 0; o < FH2; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        b01[o] = __ffma2_rn(ww[k], u01, b01[o]);
-                        b23[o] = __ffma2_rn(ww[k], u23, b23[o]);
-                        b4[o] = __fmaf_rn(ww[k].x, u4, b4[o]);
+                        a[o] = __ffma2_rn(tap(k), t, a[o]);
+                        d[o] = __ffma2_rn(tap(k), u, d[o]);
+                        e[o] = __fmaf_rn(tap(k).x, q, e[o]);
                     }
                 }
-                const int gx = ox + co;
 #pragma unroll
-                for (int o = 0; o < V2; ++o) {
-                    const int ro = r0 + o, gy = oy + ro;
-                    if (gx >= w || gy >= h) continue;
-                    const int ri = (ro + 2 * LR) * RG + (co + 2 * LR);
-                    const float x = in_x[ri], y = in_y[ri];
-                    const float grad = b01[o].x + y * b01[o].y - b23[o].y + 2.0f * x * b23[o].x - 2.0f * b4[o];
-                    const float d = x - y;
-                    l1_local += fabsf(d);
-                    const float sg = (d != d) ? d : copysignf(1.0f, d);
-                    float g = (1.0f - lambda) * sg / m_total;
-                    g += -lambda * grad / m_total;
-                    dl[(pb + (size_t)gy * w + gx) * 3 + ch] = g;
+                for (int o = 0; o < FH2; ++o) {
+                    g01[rm * FGS + c0 + o] = a[o];
+                    g23[rm * FGS + c0 + o] = d[o];
+                    g4[rm * FGS + c0 + o] = e[o];
                 }
             }
             __syncthreads();
+            // the maps are read: the next channel's region may take their place
+            if (ch < 2) load(ch + 1);
+            // pass 4: vertical blur -> gradient, combined with the L1 term
+            for (int it = tid; it < LT * (LT / FV2); it += FL_THREADS) {
+                const int co = it % LT, r0 = (it / LT) * FV2;
+                const int gx = ox + co, gy0 = oy + r0;
+                const ptrdiff_t p0 = (ptrdiff_t)gy0 * w + gx;
+                float x[FV2], y[FV2];
+#pragma unroll
+                for (int o = 0; o < FV2; ++o) {
+                    const bool ok = gx < w && gy0 + o < h;
+                    x[o] = ok ? img[(p0 + (ptrdiff_t)o * w) * 3 + ch] : 0.0f;
+                    y[o] = ok ? tgt[(p0 + (ptrdiff_t)o * w) * 4 + ch] : 0.0f;
+                }
+                float2 a[FV2], g[FV2];
+                float e[FV2];
+#pragma unroll
+                for (int o = 0; o < FV2; ++o) {
+                    a[o] = g[o] = f2(0.0f, 0.0f);
+                    e[o] = 0.0f;
+                }
+#pragma unroll
+                for (int j = 0; j < FV2 + 10; ++j) {
+                    const int p = (r0 + j) * FGS + co;
+                    const float2 t = g01[p], u = g23[p];
+                    const float q = g4[p];
+#pragma unroll
+                    for (int o = 0; o < FV2; ++o) {
+                        const int k = j - o;
+                        if (k < 0 || k > 10) continue;
+                        a[o] = __ffma2_rn(tap(k), t, a[o]);
+                        g[o] = __ffma2_rn(tap(k), u, g[o]);
+                        e[o] = __fmaf_rn(tap(k).x, q, e[o]);
+                    }
+                }
+#pragma unroll
+                for (int o = 0; o < FV2; ++o) {
+                    if (gx >= w || gy0 + o >= h) continue;
+                    const float grad = a[o].x + y[o] * a[o].y - g[o].y + 2.0f * x[o] * g[o].x - 2.0f * e[o];
+                    const float d = x[o] - y[o];
+                    l1_local += fabsf(d);
+                    const float sg = (d != d) ? d : copysignf(1.0f, d);
+                    grad_out[(p0 + (ptrdiff_t)o * w) * 3 + ch] = g_l1 * sg + -lambda * grad / m_total;
+                }
+            }
         }
-        float l1s = block_sum_fixed(l1_local, s_red);
-        float sss = block_sum_fixed(ssim_local, s_red + LOSS_THREADS / 32);
+        float l1s = fl_block_sum(l1_local, s_red);
+        float sss = fl_block_sum(ssim_local, s_red + FL_WARPS);
         if (tid == 0) {
             partials[(size_t)blk * 2 + 0] = l1s;
             partials[(size_t)blk * 2 + 1] = sss;
         }
-        __syncthreads();
     }
 }
 
@@ -571,7 +617,7 @@ cudaError_t prepare_loss_kernel() {
     if (ready[dev]) return cudaSuccess;
     e = cudaFuncSetAttribute(k_loss, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOSS_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_loss_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOSS_SMEM);
+        e = cudaFuncSetAttribute(k_loss_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL_SMEM);
     if (e == cudaSuccess) ready[dev] = true;
     return e;
 }
@@ -581,13 +627,12 @@ cudaError_t launch_loss(const DevCam* cams, int nviews, int total_blocks, const 
     cudaError_t e = prepare_loss_kernel();
     if (e != cudaSuccess) return e;
     const int sms = device_sm_count();
-    int grid = total_dev ? sms * 2 : (total_blocks < sms * 2 ? total_blocks : sms * 2);
-    if (grid < 1) grid = 1;
+    const int most = sms * 2;
+    const int grid = std::max(1, total_dev ? most : std::min(total_blocks, most));
     if (exact)
         k_loss<<<grid, LOSS_THREADS, LOSS_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda, dl, partials);
     else
-        k_loss_fused<<<grid, LOSS_THREADS, LOSS_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda, dl,
-                                                            partials);
+        k_loss_fused<<<grid, FL_THREADS, FL_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda, dl, partials);
     if (nviews > 0) k_loss_finalize<<<nviews, FIN_THREADS, 0, st>>>(cams, nviews, partials, lambda, losses);
     return cudaGetLastError();
 }
