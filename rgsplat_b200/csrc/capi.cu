@@ -364,7 +364,7 @@ int upload_gaussians(rgs_ctx* ctx, Scene& s, const float* g, size_t n) {
     s.n = (int)n;
     if (n == 0) return RGS_OK;
     CK(ctx->stage_a.ensure(n * NP * sizeof(float)));
-    CK(cudaMemcpyAsync(ctx->stage_a.p, g, n * NP * sizeof(float), cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->stage_a.p, g, n * NP * sizeof(float), ctx->st));
     launch_aos_to_planes(ctx->stage_a.as<float>(), s.params.as<float4>(), (int)n, s.cap, ctx->st);
     CK(cudaGetLastError());
     return RGS_OK;
@@ -679,7 +679,7 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
     mark(ctx, 6);
     CK(cudaGetLastError());
     if (rgb_host) {
-        CK(cudaMemcpyAsync(rgb_host, ctx->rgb.p, px * 3 * 4, cudaMemcpyDeviceToHost, st));
+        CK(copy_to_host(rgb_host, ctx->rgb.p, px * 3 * 4, st));
         if ((rc = read_scalars(ctx))) return rc;
     }
     if (!do_backward) return RGS_OK;
@@ -784,6 +784,7 @@ int rgs_create(const rgs_options* opts, rgs_ctx** out) {
     if (o.device < 0 || o.device >= ndev) return RGS_ERR_INVALID_ARG;
     if (o.batch_pair_limit == 0) o.batch_pair_limit = BATCH_PAIR_LIMIT;
     rgs_ctx* ctx = new rgs_ctx();
+    host_copy_user(1);
     ctx->opt = o;
     ctx->device = o.device;
     t_mem = &ctx->mem;
@@ -844,6 +845,7 @@ void rgs_destroy(rgs_ctx* ctx) {
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     t_mem = nullptr;
     delete ctx;
+    host_copy_user(-1);
 }
 
 const char* rgs_last_error(const rgs_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
@@ -912,7 +914,7 @@ int rgs_render_and_backward(rgs_ctx* ctx, const float* gaussians, size_t n, cons
     if ((rc = check_finite(ctx, s))) return rc;
     size_t px = (size_t)camera->width * camera->height;
     CK(ctx->target_stage.ensure(px * 4 * 4));
-    CK(cudaMemcpyAsync(ctx->target_stage.p, target_rgba, px * 16, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->target_stage.p, target_rgba, px * 16, ctx->st));
     ctx->stats = rgs_stats{};
     float loss = 0.0f;
     if ((rc = run_view_plain(ctx, s, dc, ctx->target_stage.as<float>(), bg, cfg->lambda_dssim, true, false, &loss, nullptr)))
@@ -921,7 +923,7 @@ int rgs_render_and_backward(rgs_ctx* ctx, const float* gaussians, size_t n, cons
     if (grads_out && n) {
         CK(ctx->stage_b.ensure(n * NG * 4));
         launch_grads_to_aos(s.grads.as<float4>(), ctx->stage_b.as<float>(), (int)n, s.cap, NG, ctx->st);
-        CK(cudaMemcpyAsync(grads_out, ctx->stage_b.p, n * NG * 4, cudaMemcpyDeviceToHost, ctx->st));
+        CK(copy_to_host(grads_out, ctx->stage_b.p, n * NG * 4, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
     }
     return RGS_OK;
@@ -944,7 +946,7 @@ int rgs_render_and_backward_variant(rgs_ctx* ctx, const float* gaussians, size_t
     if ((rc = check_finite(ctx, s))) return rc;
     size_t px = (size_t)camera->width * camera->height;
     CK(ctx->target_stage.ensure(px * 4 * 4));
-    CK(cudaMemcpyAsync(ctx->target_stage.p, target_rgba, px * 16, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->target_stage.p, target_rgba, px * 16, ctx->st));
     ctx->stats = rgs_stats{};
     BwdStudy study;
     study.store_all = variant == RGS_BACKWARD_STORE_ALL;
@@ -969,7 +971,7 @@ int rgs_render_and_backward_variant(rgs_ctx* ctx, const float* gaussians, size_t
     if (grads_out && n) {
         CK(ctx->stage_b.ensure(n * NG * 4));
         launch_grads_to_aos(s.grads.as<float4>(), ctx->stage_b.as<float>(), (int)n, s.cap, NG, ctx->st);
-        CK(cudaMemcpyAsync(grads_out, ctx->stage_b.p, n * NG * 4, cudaMemcpyDeviceToHost, ctx->st));
+        CK(copy_to_host(grads_out, ctx->stage_b.p, n * NG * 4, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
     }
     return RGS_OK;
@@ -1003,7 +1005,7 @@ int rasterize_scene(rgs_ctx* ctx, Scene& s, const rgs_camera* camera, const floa
     launch_pack_framebuffer(ctx->rgb.as<float>(), ctx->final_t.as<float>(), px, format == RGS_FB_RGBA8_SRGB ? 1 : 0,
                             ctx->stage_a.p, ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, ctx->stage_a.p, bytes, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_a.p, bytes, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1042,8 +1044,8 @@ int rgs_photometric_loss_grad(rgs_ctx* ctx, const float* rendered_rgb, const flo
     assign_bases(&dc, 1, px, tiles, lb);
     if ((rc = ensure_work(ctx, 1, px, tiles, lb, 1))) return rc;
     CK(ctx->target_stage.ensure(px * 16));
-    CK(cudaMemcpyAsync(ctx->target_stage.p, target_rgba, px * 16, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(ctx->rgb.p, rendered_rgb, px * 12, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->target_stage.p, target_rgba, px * 16, ctx->st));
+    CK(copy_from_host(ctx->rgb.p, rendered_rgb, px * 12, ctx->st));
     dc.target = ctx->target_stage.as<float>();
     DevCam* cams_dev;
     if ((rc = upload_single_cam(ctx, dc, &cams_dev))) return rc;
@@ -1052,7 +1054,7 @@ int rgs_photometric_loss_grad(rgs_ctx* ctx, const float* rendered_rgb, const flo
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, ctx->st));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(loss_out, losses_dev, 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(dl_out, ctx->dl.p, px * 12, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(dl_out, ctx->dl.p, px * 12, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1071,12 +1073,12 @@ int rgs_adam_step(rgs_ctx* ctx, float* gaussians, size_t n, const float* grads, 
     if ((rc = ensure_moments(ctx, s, (int)n))) return rc;
     cudaStream_t st = ctx->st;
     CK(ctx->stage_b.ensure(n * NG * 4));
-    CK(cudaMemcpyAsync(ctx->stage_b.p, grads, n * NG * 4, cudaMemcpyHostToDevice, st));
+    CK(copy_from_host(ctx->stage_b.p, grads, n * NG * 4, st));
     launch_aos_to_grad_planes(ctx->stage_b.as<float>(), s.grads.as<float4>(), (int)n, s.cap, NG, st);
     CK(ctx->stage_c.ensure(n * NP * 4));
     CK(ctx->stage_d.ensure(n * NP * 4));
-    CK(cudaMemcpyAsync(ctx->stage_c.p, state->m1, n * NP * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->stage_d.p, state->m2, n * NP * 4, cudaMemcpyHostToDevice, st));
+    CK(copy_from_host(ctx->stage_c.p, state->m1, n * NP * 4, st));
+    CK(copy_from_host(ctx->stage_d.p, state->m2, n * NP * 4, st));
     launch_aos_to_grad_planes(ctx->stage_c.as<float>(), s.m1.as<float4>(), (int)n, s.mcap, NP, st);
     launch_aos_to_grad_planes(ctx->stage_d.as<float>(), s.m2.as<float4>(), (int)n, s.mcap, NP, st);
     CK(cudaMemcpyAsync(s.accum.p, state->grad_accum, n * 4, cudaMemcpyHostToDevice, st));
@@ -1090,9 +1092,9 @@ int rgs_adam_step(rgs_ctx* ctx, float* gaussians, size_t n, const float* grads, 
     launch_planes_to_aos(s.params.as<float4>(), ctx->stage_a.as<float>(), (int)n, s.cap, st);
     launch_grads_to_aos(s.m1.as<float4>(), ctx->stage_c.as<float>(), (int)n, s.mcap, NP, st);
     launch_grads_to_aos(s.m2.as<float4>(), ctx->stage_d.as<float>(), (int)n, s.mcap, NP, st);
-    CK(cudaMemcpyAsync(gaussians, ctx->stage_a.p, n * NP * 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(state->m1, ctx->stage_c.p, n * NP * 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(state->m2, ctx->stage_d.p, n * NP * 4, cudaMemcpyDeviceToHost, st));
+    CK(copy_to_host(gaussians, ctx->stage_a.p, n * NP * 4, st));
+    CK(copy_to_host(state->m1, ctx->stage_c.p, n * NP * 4, st));
+    CK(copy_to_host(state->m2, ctx->stage_d.p, n * NP * 4, st));
     CK(cudaMemcpyAsync(state->grad_accum, s.accum.p, n * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(state->grad_denom, s.denom.p, n * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1128,7 +1130,7 @@ int rgs_densify_and_prune(rgs_ctx* ctx, const float* gaussians, size_t n, const 
     if ((size_t)n_new > out_cap || (!out && n_new)) return fail(ctx, RGS_ERR_CAPACITY, "output buffer too small");
     CK(ctx->stage_a.ensure((size_t)n_new * NP * 4 + 4));
     launch_planes_to_aos(ctx->dens_out.as<float4>(), ctx->stage_a.as<float>(), n_new, ocap, st);
-    CK(cudaMemcpyAsync(out, ctx->stage_a.p, (size_t)n_new * NP * 4, cudaMemcpyDeviceToHost, st));
+    CK(copy_to_host(out, ctx->stage_a.p, (size_t)n_new * NP * 4, st));
     CK(cudaStreamSynchronize(st));
     return RGS_OK;
 }
@@ -1142,7 +1144,7 @@ int rgs_reset_opacities(rgs_ctx* ctx, float* gaussians, size_t n) {
     if ((rc = upload_gaussians(ctx, s, gaussians, n))) return rc;
     launch_reset_opacities(s.params.as<float4>(), (int)n, s.cap, ctx->st);
     launch_planes_to_aos(s.params.as<float4>(), ctx->stage_a.as<float>(), (int)n, s.cap, ctx->st);
-    CK(cudaMemcpyAsync(gaussians, ctx->stage_a.p, n * NP * 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(gaussians, ctx->stage_a.p, n * NP * 4, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1166,8 +1168,8 @@ int rgs_project(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_camera
     launch_project_wgsl(s.params.as<float4>(), (int)n, s.cap, cams_dev, mode == RGS_PROJECT_CPU_MATH ? 1 : 0,
                         ctx->stage_b.as<float>(), ctx->stage_c.as<uint32_t>(), ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(splats_out, ctx->stage_b.p, n * 40, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(keys_out, ctx->stage_c.p, n * 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(splats_out, ctx->stage_b.p, n * 40, ctx->st));
+    CK(copy_to_host(keys_out, ctx->stage_c.p, n * 4, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1201,7 +1203,7 @@ int rgs_gpu_render(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs_cam
     fa.empty_tile_black = 0;
     launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(rgb_out, ctx->rgb.p, px * 12, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(rgb_out, ctx->rgb.p, px * 12, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1239,7 +1241,7 @@ int rgs_trainer_get_gaussians(rgs_ctx* ctx, float* out, size_t cap, size_t* n_ou
     if (s.n == 0) return RGS_OK;
     CK(ctx->stage_a.ensure((size_t)s.n * NP * 4));
     launch_planes_to_aos(s.params.as<float4>(), ctx->stage_a.as<float>(), s.n, s.cap, ctx->st);
-    CK(cudaMemcpyAsync(out, ctx->stage_a.p, (size_t)s.n * NP * 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_a.p, (size_t)s.n * NP * 4, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1265,7 +1267,7 @@ int rgs_trainer_set_target(rgs_ctx* ctx, size_t index, const float* target_rgba)
     if (index >= ctx->cams.size() || !target_rgba) return fail(ctx, RGS_ERR_INVALID_ARG, "bad camera index or null target");
     size_t px = (size_t)ctx->cams[index].width * ctx->cams[index].height;
     CK(ctx->targets[index].ensure(px * 16));
-    CK(cudaMemcpyAsync(ctx->targets[index].p, target_rgba, px * 16, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->targets[index].p, target_rgba, px * 16, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1325,7 +1327,7 @@ int save_model(rgs_ctx* ctx, Scene& s, const char* path, bool ply) {
     else launch_pack_splat(s.params.as<float4>(), s.n, s.cap, ctx->stage_b.p, ctx->st);
     CK(cudaGetLastError());
     std::vector<uint8_t> host(bytes);
-    if (bytes) CK(cudaMemcpyAsync(host.data(), ctx->stage_b.p, bytes, cudaMemcpyDeviceToHost, ctx->st));
+    if (bytes) CK(copy_to_host(host.data(), ctx->stage_b.p, bytes, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return write_file(ctx, path, ply ? ply_header(n) : std::string(), host.data(), bytes);
 }
@@ -1346,7 +1348,7 @@ int load_model(rgs_ctx* ctx, Scene& s, const std::vector<uint8_t>& d, const PlyL
     const size_t fbytes = L.fields.size() * sizeof(PlyField);
     CK(ctx->stage_c.ensure(std::max<size_t>(body, 16)));
     CK(ctx->stage_d.ensure(std::max<size_t>(fbytes, 16)));
-    if (body) CK(cudaMemcpyAsync(ctx->stage_c.p, d.data() + L.body, body, cudaMemcpyHostToDevice, ctx->st));
+    if (body) CK(copy_from_host(ctx->stage_c.p, d.data() + L.body, body, ctx->st));
     if (fbytes) CK(cudaMemcpyAsync(ctx->stage_d.p, L.fields.data(), fbytes, cudaMemcpyHostToDevice, ctx->st));
     launch_unpack_ply(ctx->stage_c.as<uint8_t>(), L.stride, (int)L.count, ctx->stage_d.as<PlyField>(), (int)L.fields.size(),
                       L.format == 1 ? 1 : 0, s.params.as<float4>(), s.cap, ctx->st);
@@ -1365,7 +1367,7 @@ int sfm_to_scene(rgs_ctx* ctx, Scene& s, const double* xyz, const uint8_t* rgb, 
     SfmScratch& w = ctx->sfm;
     CK(w.xyz.ensure(n * 24));
     CK(w.rgb.ensure(n * 3 + 16));
-    CK(cudaMemcpyAsync(w.xyz.p, xyz, n * 24, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(w.xyz.p, xyz, n * 24, ctx->st));
     CK(cudaMemcpyAsync(w.rgb.p, rgb, n * 3, cudaMemcpyHostToDevice, ctx->st));
     int bad = 0;
     cudaError_t e = cudaSuccess;
@@ -1748,7 +1750,7 @@ int rgs_load_ply(rgs_ctx* ctx, const char* path, float* out, size_t cap, size_t*
     CK(ctx->stage_a.ensure(L.count * NP * sizeof(float)));
     launch_planes_to_aos(s.params.as<float4>(), ctx->stage_a.as<float>(), s.n, s.cap, ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, ctx->stage_a.p, L.count * NP * sizeof(float), cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_a.p, L.count * NP * sizeof(float), ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1763,7 +1765,7 @@ int rgs_gaussians_from_sfm(rgs_ctx* ctx, const double* xyz, const uint8_t* rgb, 
     CK(ctx->stage_a.ensure(n * NP * sizeof(float)));
     launch_planes_to_aos(s.params.as<float4>(), ctx->stage_a.as<float>(), s.n, s.cap, ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, ctx->stage_a.p, n * NP * sizeof(float), cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_a.p, n * NP * sizeof(float), ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1803,10 +1805,10 @@ int rgs_srgb8_to_linear(rgs_ctx* ctx, const uint8_t* rgba8, size_t npix, float* 
     if (npix == 0) return RGS_OK;
     CK(ctx->stage_a.ensure(npix * 4));
     CK(ctx->stage_b.ensure(npix * 16));
-    CK(cudaMemcpyAsync(ctx->stage_a.p, rgba8, npix * 4, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->stage_a.p, rgba8, npix * 4, ctx->st));
     launch_srgb8_to_linear(ctx->stage_a.p, npix, ctx->stage_b.as<float>(), ctx->st);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, ctx->stage_b.p, npix * 16, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_b.p, npix * 16, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -1818,7 +1820,7 @@ int rgs_trainer_set_target_rgba8(rgs_ctx* ctx, size_t index, const uint8_t* rgba
     const size_t px = (size_t)ctx->cams[index].width * ctx->cams[index].height;
     CK(ctx->targets[index].ensure(px * 16));
     CK(ctx->stage_a.ensure(std::max<size_t>(px * 4, 16)));
-    CK(cudaMemcpyAsync(ctx->stage_a.p, rgba8, px * 4, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->stage_a.p, rgba8, px * 4, ctx->st));
     launch_srgb8_to_linear(ctx->stage_a.p, px, ctx->targets[index].as<float>(), ctx->st);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->st));
@@ -1989,7 +1991,7 @@ int rgs_trainer_get_grads(rgs_ctx* ctx, float* out) {
     if (!out) return fail(ctx, RGS_ERR_INVALID_ARG, "null argument");
     CK(ctx->stage_b.ensure((size_t)s.n * NG * 4));
     launch_grads_to_aos(s.grads.as<float4>(), ctx->stage_b.as<float>(), s.n, s.cap, NG, ctx->st);
-    CK(cudaMemcpyAsync(out, ctx->stage_b.p, (size_t)s.n * NG * 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(out, ctx->stage_b.p, (size_t)s.n * NG * 4, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return RGS_OK;
 }
@@ -2079,8 +2081,8 @@ int rgs_trainer_get_adam_state(rgs_ctx* ctx, rgs_adam_state* state) {
     CK(ctx->stage_d.ensure(len * NP * 4));
     launch_grads_to_aos(s.m1.as<float4>(), ctx->stage_c.as<float>(), (int)len, s.mcap, NP, ctx->st);
     launch_grads_to_aos(s.m2.as<float4>(), ctx->stage_d.as<float>(), (int)len, s.mcap, NP, ctx->st);
-    CK(cudaMemcpyAsync(state->m1, ctx->stage_c.p, len * NP * 4, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(state->m2, ctx->stage_d.p, len * NP * 4, cudaMemcpyDeviceToHost, ctx->st));
+    CK(copy_to_host(state->m1, ctx->stage_c.p, len * NP * 4, ctx->st));
+    CK(copy_to_host(state->m2, ctx->stage_d.p, len * NP * 4, ctx->st));
     CK(cudaMemcpyAsync(state->grad_accum, s.accum.p, len * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(state->grad_denom, s.denom.p, len * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
@@ -2100,8 +2102,8 @@ int rgs_trainer_set_adam_state(rgs_ctx* ctx, const rgs_adam_state* state) {
     if (!state->m1 || !state->m2 || !state->grad_accum || !state->grad_denom) return fail(ctx, RGS_ERR_INVALID_ARG, "null array");
     CK(ctx->stage_c.ensure(len * NP * 4));
     CK(ctx->stage_d.ensure(len * NP * 4));
-    CK(cudaMemcpyAsync(ctx->stage_c.p, state->m1, len * NP * 4, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(ctx->stage_d.p, state->m2, len * NP * 4, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->stage_c.p, state->m1, len * NP * 4, ctx->st));
+    CK(copy_from_host(ctx->stage_d.p, state->m2, len * NP * 4, ctx->st));
     launch_aos_to_grad_planes(ctx->stage_c.as<float>(), s.m1.as<float4>(), (int)len, s.mcap, NP, ctx->st);
     launch_aos_to_grad_planes(ctx->stage_d.as<float>(), s.m2.as<float4>(), (int)len, s.mcap, NP, ctx->st);
     CK(cudaMemcpyAsync(s.accum.p, state->grad_accum, len * 4, cudaMemcpyHostToDevice, ctx->st));
@@ -2253,7 +2255,7 @@ int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs
     size_t px, tiles, lb;
     if ((rc = debug_bin(ctx, gaussians, n, camera, dc, &cams_dev, b, px, tiles, lb))) return rc;
     CK(ctx->target_stage.ensure(px * 16));
-    CK(cudaMemcpyAsync(ctx->target_stage.p, target_rgba, px * 16, cudaMemcpyHostToDevice, ctx->st));
+    CK(copy_from_host(ctx->target_stage.p, target_rgba, px * 16, ctx->st));
     dc.target = ctx->target_stage.as<float>();
     if ((rc = upload_single_cam(ctx, dc, &cams_dev))) return rc;
     BlendArgs fa = blend_args(ctx, ctx->sc, cams_dev, 1, nullptr, tiles, b, bg, true);

@@ -1,0 +1,218 @@
+// hostcopy.cu -- large copies between device memory and the caller's pageable
+// host arrays (Gaussians, gradients, moments, images).
+//
+// cudaMemcpyAsync on pageable memory goes through the driver's staging buffers
+// on the calling thread, which also takes every page fault of a fresh
+// destination: 4.9 GB/s into a newly allocated array. Here several threads claim
+// chunks in turn; each copies its chunk between the caller's array and one of
+// its two page-locked slabs while the other slab is on the bus, so both the
+// memory copies and the page faults run in parallel. Measured on a 16-core host,
+// before and after: reading a scene of 47 MB 9.9 -> 2.9 ms, 236 MB 48 -> 11.7 ms
+// (20 GB/s); writing one 2.6 -> 1.5, 21 -> 5.8 ms. HOST_COPY_MIN lies where the
+// threads' start is paid back: 6.1 MB read 0.84 -> 0.78 ms but written 0.38 ->
+// 0.47, 8.4 MB 1.1 -> 1.2 and 0.51 -> 0.54, 9.4 MB 1.23 -> 0.86 and 0.60 -> 0.48.
+//
+// The slabs belong to the process, not to a context: at most HC_SLABS of them,
+// page-locked when first needed (page-locking is slow, so it is not paid again
+// by every context), handed out under a mutex, and freed when the last context is
+// destroyed. A copy that finds none free, or whose threads cannot be started,
+// falls back to the plain copy.
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "rgs_internal.cuh"
+
+namespace rgs {
+
+namespace {
+
+constexpr size_t HC_CHUNK = 1 << 20;
+constexpr int HC_THREADS = 8;
+constexpr int HC_SLABS = 2 * HC_THREADS;
+
+struct Pool {
+    std::mutex mu;
+    std::vector<void*> idle;
+    int made = 0, users = 0;
+};
+Pool& pool() {
+    static Pool* p = new Pool;  // outlives static destruction: contexts may too
+    return *p;
+}
+
+// Up to n slabs (an even number).
+std::vector<void*> take(int n) {
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    std::vector<void*> got;
+    got.reserve((size_t)n);
+    p.idle.reserve(HC_SLABS);  // nothing below allocates
+    while ((int)got.size() < n) {
+        if (!p.idle.empty()) {
+            got.push_back(p.idle.back());
+            p.idle.pop_back();
+            continue;
+        }
+        void* s = nullptr;
+        if (p.made == HC_SLABS || cudaHostAlloc(&s, HC_CHUNK, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
+        ++p.made;
+        got.push_back(s);
+    }
+    if (got.size() % 2) {
+        p.idle.push_back(got.back());
+        got.pop_back();
+    }
+    return got;
+}
+
+void free_idle(Pool& p) {
+    for (void* s : p.idle) cudaFreeHost(s);
+    p.made -= (int)p.idle.size();
+    p.idle.clear();
+}
+
+void give(const std::vector<void*>& slabs) {
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    for (void* s : slabs) p.idle.push_back(s);
+    if (p.users == 0) free_idle(p);
+}
+
+struct Job {
+    char* host;
+    char* dev;
+    size_t bytes;
+    bool to_host;
+    cudaStream_t st;
+    int device;
+    std::atomic<size_t> next{0};
+    std::atomic<int> err{(int)cudaSuccess};
+
+    void failed(cudaError_t e) {
+        int ok = (int)cudaSuccess;
+        if (e != cudaSuccess) err.compare_exchange_strong(ok, (int)e);
+    }
+    // Claims a chunk; false when none is left or a thread failed.
+    bool claim(size_t& off, size_t& len) {
+        off = next.fetch_add(1) * HC_CHUNK;
+        if (off >= bytes || err.load() != (int)cudaSuccess) return false;
+        len = std::min(HC_CHUNK, bytes - off);
+        return true;
+    }
+    void run(void* slab0, void* slab1) {
+        void* slab[2] = {slab0, slab1};
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        cudaError_t e = cudaSetDevice(device);
+        for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
+        failed(e);
+        if (e == cudaSuccess) {
+            if (to_host) receive(slab, ev);
+            else send(slab, ev);
+        }
+        for (cudaEvent_t v : ev)
+            if (v) cudaEventDestroy(v);
+    }
+    void receive(void* const slab[2], const cudaEvent_t ev[2]) {
+        size_t off[2] = {0, 0}, len[2] = {0, 0};
+        bool live[2] = {false, false};
+        auto issue = [&](int b) {
+            live[b] = claim(off[b], len[b]);
+            if (!live[b]) return;
+            cudaError_t e = cudaMemcpyAsync(slab[b], dev + off[b], len[b], cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
+            failed(e);
+            live[b] = e == cudaSuccess;
+        };
+        issue(0);
+        for (int b = 0; live[b]; b ^= 1) {
+            issue(b ^ 1);
+            const cudaError_t e = cudaEventSynchronize(ev[b]);
+            failed(e);
+            if (e == cudaSuccess) std::memcpy(host + off[b], slab[b], len[b]);
+        }
+    }
+    void send(void* const slab[2], const cudaEvent_t ev[2]) {
+        bool used[2] = {false, false};
+        size_t off, len;
+        for (int b = 0; claim(off, len); b ^= 1) {
+            cudaError_t e = used[b] ? cudaEventSynchronize(ev[b]) : cudaSuccess;
+            if (e == cudaSuccess) {
+                std::memcpy(slab[b], host + off, len);
+                e = cudaMemcpyAsync(dev + off, slab[b], len, cudaMemcpyHostToDevice, st);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
+            used[b] = e == cudaSuccess;
+            failed(e);
+        }
+        // the slabs go back to the pool: wait for what is still on the bus
+        for (int b = 0; b < 2; ++b)
+            if (used[b]) failed(cudaEventSynchronize(ev[b]));
+    }
+};
+
+cudaError_t host_copy(void* host, void* dev, size_t bytes, bool to_host, cudaStream_t st) {
+    const auto plain = [&] {
+        return to_host ? cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st)
+                       : cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
+    };
+    if (bytes < HOST_COPY_MIN) return plain();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        cudaGetLastError();
+        return plain();
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return plain();  // page-locked already
+    const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
+    const int want = std::min({HC_THREADS, cores, (int)(bytes / (2 * HC_CHUNK))});
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::vector<void*> slabs;
+    std::vector<std::thread> threads;
+    Job job;
+    job.host = (char*)host;
+    job.dev = (char*)dev;
+    job.bytes = bytes;
+    job.to_host = to_host;
+    job.st = st;
+    job.device = device;
+    try {
+        threads.reserve((size_t)want);
+        slabs = take(2 * want);
+        // fewer threads than asked for do the same work
+        for (size_t k = 2; k + 1 < slabs.size(); k += 2) threads.emplace_back(&Job::run, &job, slabs[k], slabs[k + 1]);
+    } catch (...) {
+    }
+    if (slabs.empty()) return plain();
+    job.run(slabs[0], slabs[1]);
+    for (std::thread& t : threads) t.join();
+    e = (cudaError_t)job.err.load();
+    if (e != cudaSuccess) cudaStreamSynchronize(st);  // no slab goes back with a copy in flight
+    give(slabs);
+    return e;
+}
+
+}  // namespace
+
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    return host_copy(dst, const_cast<void*>(src), bytes, true, st);
+}
+cudaError_t copy_from_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    return host_copy(const_cast<void*>(src), dst, bytes, false, st);
+}
+
+void host_copy_user(int add) {
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    p.users += add;
+    if (p.users == 0) free_idle(p);
+}
+
+}  // namespace rgs

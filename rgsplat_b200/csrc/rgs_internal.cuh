@@ -153,6 +153,16 @@ struct SfmScratch {
 // device.cu: SM count of the current device, cached per device ordinal.
 int device_sm_count();
 
+// hostcopy.cu: copies with the caller's host arrays, ordered on st. Pageable
+// arrays of at least HOST_COPY_MIN bytes are copied by several threads through
+// page-locked slabs and the call returns when the copy is done; others are
+// cudaMemcpyAsync. host_copy_user(+1 / -1): a context comes or goes (the slabs
+// are freed with the last).
+constexpr size_t HOST_COPY_MIN = 8 << 20;
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
+cudaError_t copy_from_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
+void host_copy_user(int add);
+
 // layout.cu
 void launch_aos_to_planes(const float* aos, float4* planes, int n, int cap, cudaStream_t st);
 void launch_planes_to_aos(const float4* planes, float* aos, int n, int cap, cudaStream_t st);
