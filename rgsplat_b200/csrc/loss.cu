@@ -13,11 +13,11 @@
 // each input pixel about once and dL/dpixel is written once. The blurs are
 // register-blocked (a thread produces a run of outputs from one sliding
 // window, so each shared-memory value and each product is formed once per run).
-// Two kernels: k_loss keeps the reference's separate multiply and add per tap and
-// its divisions (dL/dpixel bit-identical, rgs_options.exact_loss); k_loss_fused,
-// the default, accumulates with fused multiply-adds on packed f32x2 pairs and
-// forms the SSIM quotients from one reciprocal. The scalar loss is reduced per
-// CTA and then per view in a fixed order (deterministic).
+// k_loss<false>, the default, accumulates with fused multiply-adds and forms the
+// SSIM quotients from one reciprocal; k_loss<true> keeps the reference's separate
+// multiply and add per tap and its divisions (dL/dpixel bit-identical,
+// rgs_options.exact_loss). The scalar loss is reduced per CTA and then per view
+// in a fixed order (deterministic).
 #include <algorithm>
 #include <mutex>
 
@@ -30,31 +30,6 @@ constexpr int LT = 32;            // output tile edge
 constexpr int LR = 5;             // window radius
 constexpr int RG = LT + 4 * LR;   // 52: staged input region
 constexpr int MG = LT + 2 * LR;   // 42: statistics / map region
-constexpr int MGP = MG + 1;       // padded row stride of the maps (odd: no bank conflicts)
-constexpr int LTP = LT + 1;       // padded row stride of the blurred maps
-constexpr int LOSS_THREADS = 256;
-// register blocking of the four separable passes: each thread produces a
-// run of outputs along the blur direction from one sliding window of inputs
-constexpr int H1 = 7;             // pass 1 (rows of x, y, x^2, y^2, xy): 6 runs per row
-constexpr int V1 = 7;             // pass 2 (columns -> statistics): 6 runs per column
-constexpr int H2 = 8;             // pass 3 (rows of the five maps): 4 runs per row
-constexpr int V2 = 4;             // pass 4 (columns -> gradient): 8 runs per column
-static_assert(MG % H1 == 0 && MG % V1 == 0 && LT % H2 == 0 && LT % V2 == 0, "run lengths must tile the regions");
-constexpr size_t LOSS_SMEM =
-    sizeof(float) * (2 * RG * RG + 5 * RG * MG + 5 * MG * MGP + 16 + 2 * LOSS_THREADS / 32);
-static_assert(5 * MG * LTP <= 5 * RG * MG, "pass-3 output must fit in the pass-1 buffer");
-
-__device__ __forceinline__ float block_sum_fixed(float v, float* s_red) {
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) s_red[w] = v;
-    __syncthreads();
-    float t = 0.0f;
-    for (int k = 0; k < LOSS_THREADS / 32; ++k) t += s_red[k];
-    return t;
-}
 
 // From the blurred statistics of one pixel (means mx, my; second moments
 // exx, eyy, exy): its SSIM value (returned) and the maps the gradient blurs
@@ -85,208 +60,10 @@ __device__ __forceinline__ float ssim_maps(float mx, float my, float exx, float 
     return s_map;
 }
 
-__global__ void __launch_bounds__(LOSS_THREADS) k_loss(const DevCam* __restrict__ cams, int nviews, const uint32_t* total_dev,
-                                                       int total_host, const float* __restrict__ rgb, float lambda,
-                                                       float* __restrict__ dl, float* __restrict__ partials) {
-    extern __shared__ float smem[];
-    float* in_x = smem;
-    float* in_y = in_x + RG * RG;
-    float* tmp = in_y + RG * RG;         // pass 1 out: [5][RG rows][MG cols]; pass 3 out: [5][MG][LTP]
-    float* st = tmp + 5 * RG * MG;        // pass 2 out (maps): [5][MG][MGP]
-    float* kw = st + 5 * MG * MGP;        // 11 taps
-    float* s_red = kw + 16;
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        // gaussian_kernel_1d(5, 1.5), backward.rs:759-772
-        float sum = 0.0f;
-        float v[11];
-        for (int i = 0; i < 11; ++i) {
-            float d = (float)i - 5.0f;
-            v[i] = exp_cr(-0.5f * d * d / (1.5f * 1.5f));
-            sum += v[i];
-        }
-        for (int i = 0; i < 11; ++i) kw[i] = v[i] / sum;
-    }
-    __syncthreads();
-    float w11[11];
-#pragma unroll
-    for (int k = 0; k < 11; ++k) w11[k] = kw[k];
-    const int total = total_dev ? (int)*total_dev : total_host;
-    for (int blk = blockIdx.x; blk < total; blk += gridDim.x) {
-        int v = 0;
-        while (v + 1 < nviews && cams[v + 1].loss_base <= blk) ++v;
-        const DevCam& c = cams[v];
-        const int w = c.width, h = c.height;
-        const int lb = blk - c.loss_base;
-        const int ox = (lb % c.loss_bx) * LT, oy = (lb / c.loss_bx) * LT;
-        const float m_total = (float)((size_t)w * h * 3);
-        const float* tgt = c.target;
-        const size_t pb = (size_t)c.pix_base;
-        float l1_local = 0.0f, ssim_local = 0.0f;
-        for (int ch = 0; ch < 3; ++ch) {
-            for (int i = tid; i < RG * RG; i += LOSS_THREADS) {
-                int r = i / RG, cc = i - r * RG;
-                int gx = ox - 2 * LR + cc, gy = oy - 2 * LR + r;
-                float xv = 0.0f, yv = 0.0f;
-                if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                    size_t p = (size_t)gy * w + gx;
-                    xv = rgb[(pb + p) * 3 + ch];
-                    yv = tgt[p * 4 + ch];
-                }
-                in_x[i] = xv;
-                in_y[i] = yv;
-            }
-            __syncthreads();
-            // pass 1: horizontal blur of x, y, x^2, y^2, xy over rows [0, RG),
-            // map columns [0, MG); a run of H1 outputs per thread
-            for (int it = tid; it < RG * (MG / H1); it += LOSS_THREADS) {
-                const int r = it / (MG / H1), c0 = (it - r * (MG / H1)) * H1;
-                const float* rx = in_x + r * RG + c0;
-                const float* ry = in_y + r * RG + c0;
-                float a[H1][5];
-#pragma unroll
-                for (int o = 0; o < H1; ++o)
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) a[o][q] = 0.0f;
-#pragma unroll
-                for (int j = 0; j < H1 + 10; ++j) {
-                    const float xk = rx[j], yk = ry[j];
-                    const float xx = xk * xk, yy = yk * yk, xy = xk * yk;
-#pragma unroll
-                    for (int o = 0; o < H1; ++o) {
-                        const int k = j - o;
-                        if (k < 0 || k > 10) continue;
-                        a[o][0] += w11[k] * xk;
-                        a[o][1] += w11[k] * yk;
-                        a[o][2] += w11[k] * xx;
-                        a[o][3] += w11[k] * yy;
-                        a[o][4] += w11[k] * xy;
-                    }
-                }
-#pragma unroll
-                for (int o = 0; o < H1; ++o)
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) tmp[q * RG * MG + r * MG + c0 + o] = a[o][q];
-            }
-            __syncthreads();
-            // pass 2: vertical blur -> statistics, then the per-pixel SSIM
-            // maps P, Q, R, Q*mu_y, R*mu_x (zero outside the image)
-            for (int it = tid; it < MG * (MG / V1); it += LOSS_THREADS) {
-                const int cm = it % MG, r0 = (it / MG) * V1;
-                float mu[V1][5];
-#pragma unroll
-                for (int o = 0; o < V1; ++o)
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) mu[o][q] = 0.0f;
-#pragma unroll
-                for (int j = 0; j < V1 + 10; ++j) {
-                    float t[5];
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) t[q] = tmp[q * RG * MG + (r0 + j) * MG + cm];
-#pragma unroll
-                    for (int o = 0; o < V1; ++o) {
-                        const int k = j - o;
-                        if (k < 0 || k > 10) continue;
-#pragma unroll
-                        for (int q = 0; q < 5; ++q) mu[o][q] += w11[k] * t[q];
-                    }
-                }
-                const int gx = ox - LR + cm;
-#pragma unroll
-                for (int o = 0; o < V1; ++o) {
-                    const int rm = r0 + o, gy = oy - LR + rm;
-                    float P = 0.0f, Q = 0.0f, R = 0.0f, QM = 0.0f, RM = 0.0f;
-                    if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                        const float s = ssim_maps<false>(mu[o][0], mu[o][1], mu[o][2], mu[o][3], mu[o][4], P, Q, R, QM, RM);
-                        if (rm >= LR && rm < LR + LT && cm >= LR && cm < LR + LT) ssim_local += s;
-                    }
-                    float* sp = st + rm * MGP + cm;
-                    sp[0 * MG * MGP] = P;
-                    sp[1 * MG * MGP] = Q;
-                    sp[2 * MG * MGP] = R;
-                    sp[3 * MG * MGP] = QM;
-                    sp[4 * MG * MGP] = RM;
-                }
-            }
-            __syncthreads();
-            // pass 3: horizontal blur of the maps: rows [0, MG), output cols [0, LT)
-            for (int it = tid; it < MG * (LT / H2); it += LOSS_THREADS) {
-                const int rm = it % MG, c0 = (it / MG) * H2;
-#pragma unroll 1
-                for (int q = 0; q < 5; ++q) {
-                    const float* row = st + q * MG * MGP + rm * MGP + c0;
-                    float a[H2];
-#pragma unroll
-                    for (int o = 0; o < H2; ++o) a[o] = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < H2 + 10; ++j) {
-                        const float t = row[j];
-#pragma unroll
-                        for (int o = 0; o < H2; ++o) {
-                            const int k = j - o;
-                            if (k < 0 || k > 10) continue;
-                            a[o] += w11[k] * t;
-                        }
-                    }
-#pragma unroll
-                    for (int o = 0; o < H2; ++o) tmp[q * MG * LTP + rm * LTP + c0 + o] = a[o];
-                }
-            }
-            __syncthreads();
-            // pass 4: vertical blur -> gradient, combined with the L1 term
-            for (int it = tid; it < LT * (LT / V2); it += LOSS_THREADS) {
-                const int co = it % LT, r0 = (it / LT) * V2;
-                float b[V2][5];
-#pragma unroll
-                for (int o = 0; o < V2; ++o)
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) b[o][q] = 0.0f;
-#pragma unroll
-                for (int j = 0; j < V2 + 10; ++j) {
-                    float t[5];
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) t[q] = tmp[q * MG * LTP + (r0 + j) * LTP + co];
-#pragma unroll
-                    for (int o = 0; o < V2; ++o) {
-                        const int k = j - o;
-                        if (k < 0 || k > 10) continue;
-#pragma unroll
-                        for (int q = 0; q < 5; ++q) b[o][q] += w11[k] * t[q];
-                    }
-                }
-                const int gx = ox + co;
-#pragma unroll
-                for (int o = 0; o < V2; ++o) {
-                    const int ro = r0 + o, gy = oy + ro;
-                    if (gx >= w || gy >= h) continue;
-                    const int ri = (ro + 2 * LR) * RG + (co + 2 * LR);
-                    const float x = in_x[ri], y = in_y[ri];
-                    const float grad = b[o][0] + y * b[o][1] - b[o][3] + 2.0f * x * b[o][2] - 2.0f * b[o][4];
-                    const float d = x - y;
-                    l1_local += fabsf(d);
-                    const float sg = (d != d) ? d : copysignf(1.0f, d);
-                    float g = (1.0f - lambda) * sg / m_total;
-                    g += -lambda * grad / m_total;
-                    dl[(pb + (size_t)gy * w + gx) * 3 + ch] = g;
-                }
-            }
-            __syncthreads();
-        }
-        float l1s = block_sum_fixed(l1_local, s_red);
-        float sss = block_sum_fixed(ssim_local, s_red + LOSS_THREADS / 32);
-        if (tid == 0) {
-            partials[(size_t)blk * 2 + 0] = l1s;
-            partials[(size_t)blk * 2 + 1] = sss;
-        }
-        __syncthreads();
-    }
-}
-
-// The same loss with fused multiply-adds, two independent accumulators per
-// packed f32x2 instruction (per lane the rounding of one fmaf): the statistics
-// as (x, y), (x^2, y^2), xy; the maps as (P, Q), (R, Q mu_y), R mu_x. Pass
-// outputs live in shared memory as float2 planes of those pairs (plus one float
-// plane).
+// Two independent accumulators per packed f32x2 instruction (per lane the
+// rounding of the scalar one): the statistics as (x, y), (x^2, y^2), xy; the maps
+// as (P, Q), (R, Q mu_y), R mu_x. Pass outputs live in shared memory as float2
+// planes of those pairs (plus one float plane).
 //
 // What bounds it: FMA issue (339 fused multiply-adds per pixel and channel with
 // the halos) and the latency around the four barriers per channel. Ten warps
@@ -297,7 +74,9 @@ __global__ void __launch_bounds__(LOSS_THREADS) k_loss(const DevCam* __restrict_
 // warp by 4-byte asynchronous copies, the next channel's while this one's last
 // pass runs; rows are padded against bank conflicts. 0.84 -> 0.77 ms (1M
 // Gaussians x 8 views, 8.5M pixels), 162 -> 151 us (1600x1064), 20.0 -> 17.5 us
-// (256x256). 256 and 384 threads 0.85 and 0.83 ms.
+// (256x256). 256 and 384 threads 0.85 and 0.83 ms. The exact form, twice the
+// operations of each tap, ran on scalars with 256 threads before: 370 -> 315 us
+// (three views, 2.75M pixels).
 //
 // Fewer blurs would do: P', (Q mu_y)' and (R mu_x)' enter the gradient as one
 // sum, and E[x^2] + E[y^2] as one; seven blurs ran 0.60 ms, eight 0.71. Not
@@ -339,10 +118,22 @@ __device__ __forceinline__ float fl_block_sum(float v, float* s_red) {
     return t;
 }
 
-__global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __restrict__ cams, int nviews,
-                                                              const uint32_t* total_dev, int total_host,
-                                                              const float* __restrict__ rgb, float lambda,
-                                                              float* __restrict__ dl, float* __restrict__ partials) {
+// acc + w * x: rounded once, or (EXACT) twice, as the reference's multiply and
+// add. `one` is 1 at run time: the compiler joins a packed multiply and add into
+// one instruction, but not a multiply and this fma.
+template <bool EXACT>
+__device__ __forceinline__ float2 tap_add2(float2 w, float2 x, float2 acc, float2 one) {
+    return EXACT ? __ffma2_rn(__fmul2_rn(w, x), one, acc) : __ffma2_rn(w, x, acc);
+}
+template <bool EXACT>
+__device__ __forceinline__ float tap_add(float w, float x, float acc) {
+    return EXACT ? __fadd_rn(acc, __fmul_rn(w, x)) : __fmaf_rn(w, x, acc);
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(FL_THREADS, 2) k_loss(const DevCam* __restrict__ cams, int nviews, const uint32_t* total_dev,
+                                                        int total_host, const float* __restrict__ rgb, float lambda, float one,
+                                                        float* __restrict__ dl, float* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char fl_smem[];
     float2* in = reinterpret_cast<float2*>(fl_smem);               // [RG][FRS]
     float2* m01 = reinterpret_cast<float2*>(fl_smem);              // [MG][FTS], over the input
@@ -373,6 +164,7 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
 #pragma unroll
     for (int k = 0; k < 6; ++k) ww[k] = f2(kw[k], kw[k]);
     auto tap = [&](int k) { return ww[k < 6 ? k : 10 - k]; };
+    const float2 one2 = f2(one, one);
     const int total = total_dev ? (int)*total_dev : total_host;
     for (int blk = blockIdx.x; blk < total; blk += gridDim.x) {
         int v = 0;
@@ -432,9 +224,9 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
                     for (int o = 0; o < FH1; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        a01[o] = __ffma2_rn(tap(k), xy, a01[o]);
-                        a23[o] = __ffma2_rn(tap(k), sp, a23[o]);
-                        a4[o] = __fmaf_rn(tap(k).x, cr, a4[o]);
+                        a01[o] = tap_add2<EXACT>(tap(k), xy, a01[o], one2);
+                        a23[o] = tap_add2<EXACT>(tap(k), sp, a23[o], one2);
+                        a4[o] = tap_add<EXACT>(tap(k).x, cr, a4[o]);
                     }
                 }
 #pragma unroll
@@ -464,9 +256,9 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
                     for (int o = 0; o < FV1; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        mu[o] = __ffma2_rn(tap(k), u, mu[o]);
-                        sq[o] = __ffma2_rn(tap(k), q, sq[o]);
-                        cr[o] = __fmaf_rn(tap(k).x, e, cr[o]);
+                        mu[o] = tap_add2<EXACT>(tap(k), u, mu[o], one2);
+                        sq[o] = tap_add2<EXACT>(tap(k), q, sq[o], one2);
+                        cr[o] = tap_add<EXACT>(tap(k).x, e, cr[o]);
                     }
                 }
                 const int gx = ox - LR + cm;
@@ -475,7 +267,7 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
                     const int rm = r0 + o, gy = oy - LR + rm;
                     float P = 0.0f, Q = 0.0f, R = 0.0f, QM = 0.0f, RM = 0.0f;
                     if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                        const float ssim = ssim_maps<true>(mu[o].x, mu[o].y, sq[o].x, sq[o].y, cr[o], P, Q, R, QM, RM);
+                        const float ssim = ssim_maps<!EXACT>(mu[o].x, mu[o].y, sq[o].x, sq[o].y, cr[o], P, Q, R, QM, RM);
                         if (rm >= LR && rm < LR + LT && cm >= LR && cm < LR + LT) ssim_local += ssim;
                     }
                     m01[rm * FTS + cm] = f2(P, Q);
@@ -503,9 +295,9 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
                     for (int o = 0; o < FH2; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        a[o] = __ffma2_rn(tap(k), t, a[o]);
-                        d[o] = __ffma2_rn(tap(k), u, d[o]);
-                        e[o] = __fmaf_rn(tap(k).x, q, e[o]);
+                        a[o] = tap_add2<EXACT>(tap(k), t, a[o], one2);
+                        d[o] = tap_add2<EXACT>(tap(k), u, d[o], one2);
+                        e[o] = tap_add<EXACT>(tap(k).x, q, e[o]);
                     }
                 }
 #pragma unroll
@@ -546,9 +338,9 @@ __global__ void __launch_bounds__(FL_THREADS, 2) k_loss_fused(const DevCam* __re
                     for (int o = 0; o < FV2; ++o) {
                         const int k = j - o;
                         if (k < 0 || k > 10) continue;
-                        a[o] = __ffma2_rn(tap(k), t, a[o]);
-                        g[o] = __ffma2_rn(tap(k), u, g[o]);
-                        e[o] = __fmaf_rn(tap(k).x, q, e[o]);
+                        a[o] = tap_add2<EXACT>(tap(k), t, a[o], one2);
+                        g[o] = tap_add2<EXACT>(tap(k), u, g[o], one2);
+                        e[o] = tap_add<EXACT>(tap(k).x, q, e[o]);
                     }
                 }
 #pragma unroll
@@ -615,9 +407,9 @@ cudaError_t prepare_loss_kernel() {
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(mu);
     if (ready[dev]) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_loss, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOSS_SMEM);
+    e = cudaFuncSetAttribute(k_loss<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_loss_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL_SMEM);
+        e = cudaFuncSetAttribute(k_loss<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL_SMEM);
     if (e == cudaSuccess) ready[dev] = true;
     return e;
 }
@@ -629,10 +421,8 @@ cudaError_t launch_loss(const DevCam* cams, int nviews, int total_blocks, const 
     const int sms = device_sm_count();
     const int most = sms * 2;
     const int grid = std::max(1, total_dev ? most : std::min(total_blocks, most));
-    if (exact)
-        k_loss<<<grid, LOSS_THREADS, LOSS_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda, dl, partials);
-    else
-        k_loss_fused<<<grid, FL_THREADS, FL_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda, dl, partials);
+    (exact ? k_loss<true> : k_loss<false>)<<<grid, FL_THREADS, FL_SMEM, st>>>(cams, nviews, total_dev, total_blocks, rgb, lambda,
+                                                                             1.0f, dl, partials);
     if (nviews > 0) k_loss_finalize<<<nviews, FIN_THREADS, 0, st>>>(cams, nviews, partials, lambda, losses);
     return cudaGetLastError();
 }

@@ -25,3 +25,18 @@ def test_fused_loss_matches_double(w, h, lam):
     want_dl = np.asarray(want_dl, np.float64).reshape(-1)
     assert np.abs(dl - want_dl).max() <= 1e-4 * np.abs(want_dl).max()
     assert abs(loss - want) <= 1e-5 * abs(want)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (3, 7), (31, 33), (32, 32), (42, 52), (65, 16), (200, 97), (1000, 640)])
+def test_exact_loss_matches_bit_for_bit(w, h):
+    """exact_loss rounds each product and each sum of dL/dpixel in the oracle's
+    order; the loss is summed in double (the oracle's float sum is serial), so its
+    bar is the one above."""
+    rng = np.random.default_rng(w * 1000 + h)
+    rendered = rng.random(w * h * 3, dtype=np.float32)
+    target = rng.random(w * h * 4, dtype=np.float32)
+    loss, dl = R.photometric_loss_grad(rendered, target, w, h, 0.2, ctx=R.Context(exact_loss=True))
+    _, want_dl = O.photometric_loss_grad(rendered, target, w, h, 0.2)
+    want, _ = O.photometric_loss_grad(rendered, target, w, h, 0.2, double=True)
+    np.testing.assert_array_equal(dl, np.asarray(want_dl, np.float32).reshape(-1))
+    assert abs(loss - want) <= 1e-5 * abs(want)
