@@ -12,17 +12,22 @@
 // threads' start is paid back: 6.1 MB read 0.84 -> 0.78 ms but written 0.38 ->
 // 0.47, 8.4 MB 1.1 -> 1.2 and 0.51 -> 0.54, 9.4 MB 1.23 -> 0.86 and 0.60 -> 0.48.
 //
-// The slabs belong to the process, not to a context: at most HC_SLABS of them,
-// page-locked when first needed (page-locking is slow, so it is not paid again
-// by every context), handed out under a mutex, and freed when the last context is
-// destroyed. A copy that finds none free, or whose threads cannot be started,
-// falls back to the plain copy.
+// The slabs belong to the process, not to a context: one block of HC_SLABS, handed
+// out under a mutex and given back when the last context is destroyed. It is
+// huge-page memory registered as a whole (16 MiB: 2 to 4 ms; sixteen cudaHostAlloc of
+// 1 MiB took 10 to 22; slabs of 512 KiB wrote 236 MB in 8.0 ms instead of 5.9). So
+// that a program that makes a context, copies a little and destroys it does not
+// pay even that, the block is made only once HC_FIRST bytes have gone by in large
+// copies. A copy that finds no slab free, or whose threads cannot be started, falls
+// back to the plain copy.
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <atomic>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <thread>
-#include <vector>
 
 #include "rgs_internal.cuh"
 
@@ -33,56 +38,70 @@ namespace {
 constexpr size_t HC_CHUNK = 1 << 20;
 constexpr int HC_THREADS = 8;
 constexpr int HC_SLABS = 2 * HC_THREADS;
+constexpr size_t HC_BLOCK = HC_SLABS * HC_CHUNK;
+constexpr size_t HC_HUGE = 2 << 20;
+constexpr size_t HC_FIRST = 32 << 20;
 
 struct Pool {
     std::mutex mu;
-    std::vector<void*> idle;
-    int made = 0, users = 0;
+    void* map = nullptr;  // the block's mapping, HC_BLOCK + HC_HUGE bytes
+    char* block = nullptr;
+    void* idle[HC_SLABS];
+    int idle_n = 0, users = 0;
+    size_t seen = 0;  // bytes of large copies while there was no block
 };
 Pool& pool() {
     static Pool* p = new Pool;  // outlives static destruction: contexts may too
     return *p;
 }
 
-// Up to n slabs (an even number).
-std::vector<void*> take(int n) {
-    Pool& p = pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    std::vector<void*> got;
-    got.reserve((size_t)n);
-    p.idle.reserve(HC_SLABS);  // nothing below allocates
-    while ((int)got.size() < n) {
-        if (!p.idle.empty()) {
-            got.push_back(p.idle.back());
-            p.idle.pop_back();
-            continue;
-        }
-        void* s = nullptr;
-        if (p.made == HC_SLABS || cudaHostAlloc(&s, HC_CHUNK, cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
-        ++p.made;
-        got.push_back(s);
+void make_block(Pool& p) {
+    void* m = mmap(nullptr, HC_BLOCK + HC_HUGE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return;
+    char* q = (char*)(((uintptr_t)m + HC_HUGE - 1) & ~(uintptr_t)(HC_HUGE - 1));
+    madvise(q, HC_BLOCK, MADV_HUGEPAGE);  // a hint: small pages do the same, slower
+    if (cudaHostRegister(q, HC_BLOCK, cudaHostRegisterPortable) != cudaSuccess) {
+        cudaGetLastError();
+        munmap(m, HC_BLOCK + HC_HUGE);
+        return;
     }
-    if (got.size() % 2) {
-        p.idle.push_back(got.back());
-        got.pop_back();
-    }
-    return got;
+    p.map = m;
+    p.block = q;
+    for (int k = 0; k < HC_SLABS; ++k) p.idle[k] = q + (size_t)k * HC_CHUNK;
+    p.idle_n = HC_SLABS;
 }
 
-void free_idle(Pool& p) {
-    for (void* s : p.idle) cudaFreeHost(s);
-    p.made -= (int)p.idle.size();
-    p.idle.clear();
+// With no context left and every slab back.
+void free_block(Pool& p) {
+    if (p.users != 0 || p.idle_n != (p.block ? HC_SLABS : 0)) return;
+    if (p.block) {
+        cudaHostUnregister(p.block);
+        munmap(p.map, HC_BLOCK + HC_HUGE);
+    }
+    p.map = nullptr;
+    p.block = nullptr;
+    p.idle_n = 0;
+    p.seen = 0;
 }
 
-void give(const std::vector<void*>& slabs) {
+// Up to n slabs (an even number) for a copy of `bytes`.
+int take(int n, size_t bytes, void** got) {
     Pool& p = pool();
     std::lock_guard<std::mutex> lock(p.mu);
-    for (void* s : slabs) p.idle.push_back(s);
-    if (p.users == 0) free_idle(p);
+    if (!p.block) {
+        p.seen += bytes;
+        if (p.seen >= HC_FIRST) make_block(p);
+    }
+    n = std::min(n, p.idle_n) & ~1;
+    for (int k = 0; k < n; ++k) got[k] = p.idle[--p.idle_n];
+    return n;
+}
+
+void give(int n, void* const* slabs) {
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    for (int k = 0; k < n; ++k) p.idle[p.idle_n++] = slabs[k];
+    free_block(p);
 }
 
 struct Job {
@@ -170,12 +189,14 @@ cudaError_t host_copy(void* host, void* dev, size_t bytes, bool to_host, cudaStr
     }
     if (at.type != cudaMemoryTypeUnregistered) return plain();  // page-locked already
     const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int want = std::min({HC_THREADS, cores, (int)(bytes / (2 * HC_CHUNK))});
+    const int want = std::min({HC_THREADS, cores, (int)(bytes >> 21)});
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    std::vector<void*> slabs;
-    std::vector<std::thread> threads;
+    void* slabs[HC_SLABS];
+    const int got = take(2 * want, bytes, slabs);
+    if (got == 0) return plain();
+    std::thread threads[HC_THREADS];
     Job job;
     job.host = (char*)host;
     job.dev = (char*)dev;
@@ -184,18 +205,15 @@ cudaError_t host_copy(void* host, void* dev, size_t bytes, bool to_host, cudaStr
     job.st = st;
     job.device = device;
     try {
-        threads.reserve((size_t)want);
-        slabs = take(2 * want);
-        // fewer threads than asked for do the same work
-        for (size_t k = 2; k + 1 < slabs.size(); k += 2) threads.emplace_back(&Job::run, &job, slabs[k], slabs[k + 1]);
-    } catch (...) {
+        for (int k = 2; k < got; k += 2) threads[k / 2] = std::thread(&Job::run, &job, slabs[k], slabs[k + 1]);
+    } catch (...) {  // fewer threads than asked for do the same work
     }
-    if (slabs.empty()) return plain();
     job.run(slabs[0], slabs[1]);
-    for (std::thread& t : threads) t.join();
+    for (std::thread& t : threads)
+        if (t.joinable()) t.join();
     e = (cudaError_t)job.err.load();
     if (e != cudaSuccess) cudaStreamSynchronize(st);  // no slab goes back with a copy in flight
-    give(slabs);
+    give(got, slabs);
     return e;
 }
 
@@ -212,7 +230,7 @@ void host_copy_user(int add) {
     Pool& p = pool();
     std::lock_guard<std::mutex> lock(p.mu);
     p.users += add;
-    if (p.users == 0) free_idle(p);
+    free_block(p);
 }
 
 }  // namespace rgs
