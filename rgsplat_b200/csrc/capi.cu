@@ -511,6 +511,7 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
     ea.total = sc + SC_STPAIRS;
     ea.total64 = (unsigned long long*)(sc + SC_STPAIRS64);
     launch_entry_scan(ea, bin_grid_blocks(S), st);
+    uint32_t entry_bound = 0;  // entries the host knows there to be at most
     if (host_count) {
         int rc = read_scalars(ctx);
         if (rc) return rc;
@@ -520,6 +521,7 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
         if (!ea.packed) CK(ctx->st_masks.ensure((size_t)ctx->pair_cap * 2));
         ctx->stats.pairs += K;
         ctx->stats.supertile_entries += KS;
+        entry_bound = (uint32_t)KS;
         // the depth order may live in the sort scratch: size it for the
         // supertile sort now, while nothing is in flight, so that sort never
         // reallocates it
@@ -540,6 +542,7 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
             }
         }
     }
+    if (!host_count) entry_bound = ctx->pair_cap;
     ea.keys = ctx->pkeys.as<uint32_t>();
     ea.vals = ctx->pvals.as<uint32_t>();
     ea.cap = ctx->pair_cap;
@@ -547,7 +550,7 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
     ea.overflow = (int*)(sc + SC_OVERFLOW);
     launch_emit_supertiles(ea, bin_grid_blocks(S), st);
     mark(ctx, 3);
-    int which2 = radix_sort_pairs(ctx->pkeys.as<uint32_t>(), ctx->pvals.as<uint32_t>(), ctx->pair_cap, sc + SC_STEFF,
+    int which2 = radix_sort_pairs(ctx->pkeys.as<uint32_t>(), ctx->pvals.as<uint32_t>(), entry_bound, sc + SC_STEFF,
                                   bits_for(std::max<size_t>(st_cap, 2)), ctx->sort, ctx->sort_grid, st, &e);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "supertile sort");
     mark(ctx, 4);

@@ -325,6 +325,154 @@ __global__ void __launch_bounds__(SORT_THREADS) k_downsweep(const uint32_t* __re
     }
 }
 
+// ---- whole sort in one cluster ---------------------------------------------
+// Small inputs: all passes in one launch of one cluster. Each CTA holds a chunk of
+// at most 8192 pairs in registers, ranks it as the downsweep does, and reads the
+// other CTAs' digit totals through distributed shared memory; the ranked pairs go
+// straight to their places (L2), and the cluster barrier ends the pass. The only
+// waits are those barriers, which every thread of every CTA reaches.
+//
+// What bounded small sorts was launches: 15 of 3 to 6 us each for a few thousand
+// keys that fill no SM. Depth and supertile sort of a 256x256 view: 10k Gaussians
+// 64 -> 28 us (call 420 -> 351), 500 Gaussians 57 -> 17 (call 356 -> 304). Above
+// that the scattered stores of eight SMs bound it: 35k 69 -> 53 us, 50k 72 -> 69,
+// 65k 74 -> 81 us of kernels but 13 launches less, so the call still gains (475 ->
+// 464 us). SS_MAX lies there, at what the registers hold.
+constexpr int SS_CTAS = 8;
+constexpr int SS_THREADS = 1024;
+constexpr int SS_WARPS = SS_THREADS / 32;
+constexpr int SS_IPT = 8;
+constexpr uint32_t SS_MAX = SS_CTAS * SS_THREADS * SS_IPT;
+constexpr int SS_ROW = 257;  // counter row stride: the four threads of a digit hit different banks
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The word at shared-memory address `p` of the cluster's CTA `rank`.
+__device__ __forceinline__ uint32_t cluster_load(const uint32_t* p, int rank) {
+    uint32_t a, x;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(x) : "r"(a) : "memory");
+    return x;
+}
+
+__global__ void __cluster_dims__(SS_CTAS, 1, 1) __launch_bounds__(SS_THREADS)
+    k_sort_cluster(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, const uint32_t* n_dev, uint32_t n_host, int bits) {
+    __shared__ uint32_t s_cnt[SS_WARPS * SS_ROW];  // per warp and digit: count, then exclusive over the warps
+    __shared__ uint32_t s_tot[256];                // this CTA's digit totals, read by the cluster
+    __shared__ uint32_t s_base[256];
+    __shared__ uint32_t s_w[SS_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int rank = (int)(blockIdx.x % SS_CTAS);
+    const uint32_t n = min(load_n(n_dev, n_host), n_host);
+    const uint32_t chunk = ((n + SS_CTAS - 1) / SS_CTAS + 31u) & ~31u;
+    const uint32_t begin = min(chunk * rank, n), end = min(begin + chunk, n);
+    const int items = (int)((chunk + SS_THREADS - 1) / SS_THREADS);  // <= SS_IPT
+    const uint32_t at = begin + (uint32_t)(w * items * 32 + lane);
+    uint32_t* ki = k0;
+    uint32_t* vi = v0;
+    uint32_t* ko = k1;
+    uint32_t* vo = v1;
+    uint32_t* cnt = s_cnt + w * SS_ROW;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    for (int shift = 0; shift < bits; shift += 8) {
+        for (int i = tid; i < SS_WARPS * SS_ROW; i += SS_THREADS) s_cnt[i] = 0;
+        uint32_t k[SS_IPT], v[SS_IPT], pos[SS_IPT];
+#pragma unroll
+        for (int i = 0; i < SS_IPT; ++i) {
+            const uint32_t p = at + i * 32;
+            const bool live = i < items && p < end;
+            // written by other SMs in the pass before: from L2
+            k[i] = live ? __ldcg(ki + p) : 0u;
+            v[i] = live ? __ldcg(vi + p) : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < SS_IPT; ++i) {
+            if (i >= items) break;  // CTA-uniform
+            const bool live = at + i * 32 < end;
+            const int d = (int)((k[i] >> shift) & 255u);
+            const unsigned peers = __match_any_sync(0xffffffffu, live ? d : 256);
+            const uint32_t before = live ? cnt[d] : 0u;
+            __syncwarp();
+            if (live && lane == __ffs(peers) - 1) cnt[d] = before + __popc(peers);
+            __syncwarp();
+            pos[i] = before + __popc(peers & lt_mask);
+        }
+        __syncthreads();
+        // four threads a digit: its counts exclusive over the warps, and their sum
+        const int d = tid >> 2, q = tid & 3;
+        {
+            uint32_t c[SS_WARPS / 4], sum = 0;
+#pragma unroll
+            for (int j = 0; j < SS_WARPS / 4; ++j) {
+                c[j] = s_cnt[(q * (SS_WARPS / 4) + j) * SS_ROW + d];
+                sum += c[j];
+            }
+            uint32_t inc = sum;
+            uint32_t y = __shfl_up_sync(0xffffffffu, inc, 1, 4);
+            if (q >= 1) inc += y;
+            y = __shfl_up_sync(0xffffffffu, inc, 2, 4);
+            if (q >= 2) inc += y;
+            uint32_t run = inc - sum;
+#pragma unroll
+            for (int j = 0; j < SS_WARPS / 4; ++j) {
+                s_cnt[(q * (SS_WARPS / 4) + j) * SS_ROW + d] = run;
+                run += c[j];
+            }
+            if (q == 3) s_tot[d] = inc;
+        }
+        cluster_barrier();
+        {
+            // the digit's total over the cluster, and over the CTAs before this one
+            uint32_t all = 0, before = 0;
+#pragma unroll
+            for (int j = 0; j < SS_CTAS / 4; ++j) {
+                const int r = q * (SS_CTAS / 4) + j;
+                const uint32_t t = cluster_load(&s_tot[d], r);
+                all += t;
+                before += r < rank ? t : 0u;
+            }
+            all += __shfl_xor_sync(0xffffffffu, all, 1);
+            all += __shfl_xor_sync(0xffffffffu, all, 2);
+            before += __shfl_xor_sync(0xffffffffu, before, 1);
+            before += __shfl_xor_sync(0xffffffffu, before, 2);
+            // exclusive over the digits: 8 in a warp, then over the 32 warps
+            uint32_t inc = all;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) s_w[w] = inc;
+            __syncthreads();
+            const uint32_t sums = s_w[lane];
+            const uint32_t prior = __reduce_add_sync(0xffffffffu, lane < w ? sums : 0u);
+            if (q == 0) s_base[d] = prior + inc - all + before;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < SS_IPT; ++i) {
+            if (i >= items) break;
+            if (at + i * 32 < end) {
+                const int dd = (int)((k[i] >> shift) & 255u);
+                const uint32_t g = s_base[dd] + cnt[dd] + pos[i];
+                ko[g] = k[i];
+                vo[g] = v[i];
+            }
+        }
+        // the pass's output is complete, and every CTA has read the totals
+        cluster_barrier();
+        uint32_t* t = ki;
+        ki = ko;
+        ko = t;
+        t = vi;
+        vi = vo;
+        vo = t;
+    }
+}
+
 int sort_grid_blocks() { return device_sm_count() * 4; }
 
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n_host, const uint32_t* n_dev, int bits, SortScratch& sc,
@@ -345,6 +493,11 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n_host, const uint
     }
     uint32_t* k[2] = {keys, sc.keys2.as<uint32_t>()};
     uint32_t* v[2] = {vals, sc.vals2.as<uint32_t>()};
+    if (n_host <= SS_MAX) {
+        k_sort_cluster<<<SS_CTAS, SS_THREADS, 0, st>>>(k[0], v[0], k[1], v[1], n_dev, n_host, bits);
+        *err = cudaGetLastError();
+        return (bits + 7) / 8 & 1;
+    }
     int cur = 0;
     int shift = 0;
     // 8-bit digits; a final pass over fewer significant bits still reads 8
