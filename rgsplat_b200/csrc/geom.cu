@@ -216,26 +216,89 @@ __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__
     gv[3 * S + s] = make_float4(mg, mb, 0.0f, 0.0f);
 }
 
-// optimizer.rs:142-147 for one element.
-__device__ __forceinline__ float adam_lane(float p, float g, float& m1, float& m2, float lr, const AdamArgs& a, float bc1,
-                                           float bc2) {
-    m1 = a.b1 * m1 + a.one_minus_b1 * g;
-    m2 = a.b2 * m2 + a.one_minus_b2 * g * g;
-    float m1h = m1 / bc1;
-    float m2h = m2 / bc2;
-    float upd = lr * m1h / (sqrtf(m2h) + a.eps);
-    return p - upd;
+// ---- Adam, optimizer.rs:142-147 --------------------------------------------
+struct AdamStep {  // the step's bias corrections and their reciprocals
+    float bc1, bc2, r1, r2;
+};
+
+__device__ __forceinline__ AdamStep adam_step(const AdamArgs& a) {
+    AdamStep s;
+    s.bc1 = a.bc_dev ? a.bc_dev[0] : a.bc1;
+    s.bc2 = a.bc_dev ? a.bc_dev[1] : a.bc2;
+    s.r1 = 1.0f / s.bc1;
+    s.r2 = 1.0f / s.bc2;
+    return s;
 }
 
-// Adam on plane p of Gaussian i (lanes 0..3; plane 2 has only three).
-// One plane's update with its moments already loaded (m1, m2 updated in place).
-__device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4& m1, float4& m2, const AdamArgs& a, float bc1,
-                                              float bc2) {
+// One element's update from its new moments, as the reference writes it.
+__device__ __forceinline__ float adam_divide(float m1, float m2, float lr, const AdamArgs& a, const AdamStep& s) {
+    const float m1h = m1 / s.bc1;
+    const float m2h = m2 / s.bc2;
+    return lr * m1h / (sqrtf(m2h) + a.eps);
+}
+
+// The same without a branch, for values in a range that `ok` reports: quotients and
+// root are one hardware approximation and one correction by the exact remainder
+// each (Markstein, IBM J. Res. Dev. 34(1), 1990: the corrected value is the
+// rounded one, save for rare cases an ulp off). 0 <= m2; m2 = 0 has root 0.
+__device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, const AdamArgs& a, const AdamStep& s, bool& ok) {
+    float q = m1 * s.r1;
+    const float m1h = __fmaf_rn(__fmaf_rn(-q, s.bc1, m1), s.r1, q);
+    q = m2 * s.r2;
+    const float m2h = __fmaf_rn(__fmaf_rn(-q, s.bc2, m2), s.r2, q);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(m2h));
+    q = m2h * y;
+    float root = __fmaf_rn(__fmaf_rn(-q, q, m2h), 0.5f * y, q);
+    const bool none = m2h == 0.0f;
+    root = none ? 0.0f : root;
+    const float num = lr * m1h, den = root + a.eps;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den));
+    y = __fmaf_rn(__fmaf_rn(-den, y, 1.0f), y, y);
+    q = num * y;
+    q = __fmaf_rn(__fmaf_rn(-den, q, num), y, q);
+    ok = ok && (none || m2h >= 0x1p-100f) && den >= 0x1p-60f && den <= 0x1p60f && fabsf(num) <= 0x1p60f;
+    return q;
+}
+
+// One plane's update with its moments already loaded (m1, m2 updated in place;
+// plane 2 has only three lanes).
+//
+// Written with the division and root alone, the pass was bound by their
+// instructions (176 an element, 79 % of the issue slots: zeros and small values
+// take the slow path of each), not by memory; a test per element around a shorter
+// form cost as much as it saved, so four elements share one. Adam alone on 1M
+// Gaussians 367 -> 266 us (1.66 GB of traffic: 6.2 TB/s, memory bound), on 200k
+// 91 -> 66; the fused step's SH half (1M, 8 views) 445 -> 284, geometry half 176 ->
+// 143.
+__device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4& m1, float4& m2, const AdamArgs& a,
+                                              const AdamStep& s) {
     const float* lr = a.lr + p * 4;
-    pv.x = adam_lane(pv.x, g.x, m1.x, m2.x, lr[0], a, bc1, bc2);
-    pv.y = adam_lane(pv.y, g.y, m1.y, m2.y, lr[1], a, bc1, bc2);
-    pv.z = adam_lane(pv.z, g.z, m1.z, m2.z, lr[2], a, bc1, bc2);
-    if (p != 2) pv.w = adam_lane(pv.w, g.w, m1.w, m2.w, lr[3], a, bc1, bc2);
+    const bool w = p != 2;
+    m1.x = a.b1 * m1.x + a.one_minus_b1 * g.x;
+    m1.y = a.b1 * m1.y + a.one_minus_b1 * g.y;
+    m1.z = a.b1 * m1.z + a.one_minus_b1 * g.z;
+    m2.x = a.b2 * m2.x + a.one_minus_b2 * g.x * g.x;
+    m2.y = a.b2 * m2.y + a.one_minus_b2 * g.y * g.y;
+    m2.z = a.b2 * m2.z + a.one_minus_b2 * g.z * g.z;
+    if (w) {
+        m1.w = a.b1 * m1.w + a.one_minus_b1 * g.w;
+        m2.w = a.b2 * m2.w + a.one_minus_b2 * g.w * g.w;
+    }
+    bool ok = true;
+    float4 u = make_float4(adam_divide_fast(m1.x, m2.x, lr[0], a, s, ok), adam_divide_fast(m1.y, m2.y, lr[1], a, s, ok),
+                           adam_divide_fast(m1.z, m2.z, lr[2], a, s, ok), 0.0f);
+    if (w) u.w = adam_divide_fast(m1.w, m2.w, lr[3], a, s, ok);
+    if (!ok) {
+        u.x = adam_divide(m1.x, m2.x, lr[0], a, s);
+        u.y = adam_divide(m1.y, m2.y, lr[1], a, s);
+        u.z = adam_divide(m1.z, m2.z, lr[2], a, s);
+        if (w) u.w = adam_divide(m1.w, m2.w, lr[3], a, s);
+    }
+    pv.x -= u.x;
+    pv.y -= u.y;
+    pv.z -= u.z;
+    if (w) pv.w -= u.w;
     if (p == 1) {
         // renormalise the quaternion (optimizer.rs:155-162)
         float nrm = sqrtf(pv.x * pv.x + pv.y * pv.y + pv.z * pv.z + pv.w * pv.w);
@@ -244,10 +307,10 @@ __device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4
     return pv;
 }
 
-__device__ __forceinline__ float4 adam_plane(int p, int i, int cap, float4 pv, float4 g, const AdamArgs& a, float bc1, float bc2) {
+__device__ __forceinline__ float4 adam_plane(int p, int i, int cap, float4 pv, float4 g, const AdamArgs& a, const AdamStep& step) {
     const size_t om = (size_t)p * a.mstride + i;
     float4 m1 = a.m1[om], m2 = a.m2[om];
-    pv = adam_update(p, pv, g, m1, m2, a, bc1, bc2);
+    pv = adam_update(p, pv, g, m1, m2, a, step);
     a.m1[om] = m1;
     a.m2[om] = m2;
     (void)cap;
@@ -269,11 +332,8 @@ __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const flo
     if (i >= n) return;
     if (MODE == 1 && a.skip_flag && *a.skip_flag) return;
     const size_t S = (size_t)n * nviews;
-    float bc1 = 0.0f, bc2 = 0.0f;
-    if (MODE == 1) {
-        bc1 = a.bc_dev ? a.bc_dev[0] : a.bc1;
-        bc2 = a.bc_dev ? a.bc_dev[1] : a.bc2;
-    }
+    AdamStep step{};
+    if (MODE == 1) step = adam_step(a);
     const float4* params = MODE == 1 ? a.params : params_in;
     const float4 p0 = params[i];
     const float pos[3] = {p0.x, p0.y, p0.z};
@@ -307,7 +367,7 @@ __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const flo
             const size_t o = (size_t)p * cap + i;
             float4 g = make_float4(shg[ch][kq * 4 + 0], shg[ch][kq * 4 + 1], shg[ch][kq * 4 + 2], shg[ch][kq * 4 + 3]);
             if (MODE == 1) {
-                a.params[o] = adam_plane(p, i, cap, a.params[o], g, a, bc1, bc2);
+                a.params[o] = adam_plane(p, i, cap, a.params[o], g, a, step);
             } else {
                 if (accumulate) {
                     const float4 old = grads[o];
@@ -373,9 +433,9 @@ __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const flo
     const float4 g1 = make_float4(d_rot[0], d_rot[1], d_rot[2], d_rot[3]);
     const float4 g2 = make_float4(d_ls[0], d_ls[1], d_ls[2], screen);
     if (MODE == 1) {
-        a.params[i] = adam_plane(0, i, cap, p0, g0, a, bc1, bc2);
-        a.params[(size_t)cap + i] = adam_plane(1, i, cap, p1, g1, a, bc1, bc2);
-        a.params[2 * (size_t)cap + i] = adam_plane(2, i, cap, p2, g2, a, bc1, bc2);
+        a.params[i] = adam_plane(0, i, cap, p0, g0, a, step);
+        a.params[(size_t)cap + i] = adam_plane(1, i, cap, p1, g1, a, step);
+        a.params[2 * (size_t)cap + i] = adam_plane(2, i, cap, p2, g2, a, step);
         a.grad_accum[i] += screen;
         a.grad_denom[i] += a.denom_inc;
     } else {
@@ -418,8 +478,7 @@ __global__ void __launch_bounds__(128, 8) k_geom_sh(int n, int cap, const DevCam
     if (a.skip_flag && *a.skip_flag) return;
     const int ch = (int)blockIdx.y;
     const size_t S = (size_t)n * nviews;
-    const float bc1 = a.bc_dev ? a.bc_dev[0] : a.bc1;
-    const float bc2 = a.bc_dev ? a.bc_dev[1] : a.bc2;
+    const AdamStep step = adam_step(a);
     const float4 p0 = a.params[i];
     const float pos[3] = {p0.x, p0.y, p0.z};
     const float* mplane = reinterpret_cast<const float*>(gv + (ch == 0 ? 2 : 3) * S);
@@ -449,7 +508,7 @@ __global__ void __launch_bounds__(128, 8) k_geom_sh(int n, int cap, const DevCam
         const int p = 3 + ch * 4 + kq;
         const size_t o = (size_t)p * cap + i;
         const float4 g = make_float4(shg[kq * 4 + 0], shg[kq * 4 + 1], shg[kq * 4 + 2], shg[kq * 4 + 3]);
-        a.params[o] = adam_plane(p, i, cap, a.params[o], g, a, bc1, bc2);
+        a.params[o] = adam_plane(p, i, cap, a.params[o], g, a, step);
     }
 }
 
@@ -480,12 +539,11 @@ __global__ void __launch_bounds__(256) k_adam(int n, int cap, const float4* __re
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (a.skip_flag && *a.skip_flag) return;
-    const float bc1 = a.bc_dev ? a.bc_dev[0] : a.bc1;
-    const float bc2 = a.bc_dev ? a.bc_dev[1] : a.bc2;
+    const AdamStep step = adam_step(a);
 #pragma unroll 1
     for (int p = 0; p < NPL; ++p) {
         const size_t o = (size_t)p * cap + i;
-        a.params[o] = adam_plane(p, i, cap, a.params[o], grads[o], a, bc1, bc2);
+        a.params[o] = adam_plane(p, i, cap, a.params[o], grads[o], a, step);
     }
     a.grad_accum[i] += grads[2 * (size_t)cap + i].w;
     a.grad_denom[i] += a.denom_inc;
