@@ -65,8 +65,9 @@ __device__ __forceinline__ float lane_of(const float4& v, int l) { return l == 0
 // (A) per (view, Gaussian) slot
 //   gv[0][s] = (d position xyz, d opacity (before the sigmoid factor))
 //   gv[1][s] = (dSigma00, dSigma01, dSigma02, dSigma11)
-//   gv[2][s] = (dSigma12, dSigma22, screen_grad_norm, mask * dcolor r)
-//   gv[3][s] = (mask * dcolor g, mask * dcolor b, 0, 0)
+//   gv[2][s] = (dSigma12, dSigma22, screen_grad_norm, 0)
+//   gv[3]    = mask * dcolor r, g, b as three planes of floats (the SH half reads
+//              one of them per thread)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__ params, int n, int cap, const DevCam* __restrict__ cams,
                                                    int nviews, const uint32_t* __restrict__ cnt, const float4* __restrict__ acc,
@@ -212,8 +213,11 @@ __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__
     }
     gv[s] = make_float4(dpos[0], dpos[1], dpos[2], a0.w);
     gv[S + s] = make_float4(dS[0], dS[1], dS[2], dS[3]);
-    gv[2 * S + s] = make_float4(dS[4], dS[5], sqrtf(asx * asx + asy * asy), mr);
-    gv[3 * S + s] = make_float4(mg, mb, 0.0f, 0.0f);
+    gv[2 * S + s] = make_float4(dS[4], dS[5], sqrtf(asx * asx + asy * asy), 0.0f);
+    float* masks = reinterpret_cast<float*>(gv + 3 * S);
+    masks[s] = mr;
+    masks[S + s] = mg;
+    masks[2 * S + s] = mb;
 }
 
 // ---- Adam, optimizer.rs:142-147 --------------------------------------------
@@ -322,8 +326,13 @@ __device__ __forceinline__ float4 adam_plane(int p, int i, int cap, float4 pv, f
 // (3..14) and PART 2 only the geometry planes (0..2) with grad_accum/denom,
 // each with fewer registers, so more warps per SM hide the memory latency.
 // PART 1 must run before PART 2: it reads the position that PART 2's Adam
-// step rewrites.
-template <int MODE, int PART = 0>
+// step rewrites. The slot counts of G views are loaded before any is used, and
+// then what those slots hold, so that a group costs two round trips to memory
+// instead of two a view (an unseen view adds zeros; the sums run in view order).
+// The gradient kernel, 1M Gaussians x 8 views: G = 1, 2, 4, 8: 208, 179, 160, 181 us;
+// the fused step's geometry half 143 -> 128 with 4. With one view the group is only
+// more code: 200k Gaussians 17.2 -> 18.8 us, so up to two views take G = 1.
+template <int MODE, int PART, int G>
 __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const float4* __restrict__ params_in, int n, int cap,
                                                     const DevCam* __restrict__ cams, int nviews, const uint32_t* __restrict__ cnt,
                                                     const float4* __restrict__ gv, float4* __restrict__ grads, int accumulate,
@@ -345,19 +354,27 @@ __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const flo
     for (int ch = 0; ch < 3; ++ch)
 #pragma unroll
         for (int k = 0; k < 16; ++k) shg[ch][k] = 0.0f;
-    for (int v = 0; v < nviews; ++v) {
-        const size_t s = (size_t)v * n + i;
-        if (cnt[s] == 0) continue;
-        const float4 m2 = gv[2 * S + s], m3 = gv[3 * S + s];
-        const float mk[3] = {m2.w, m3.x, m3.y};
-        if (mk[0] == 0.0f && mk[1] == 0.0f && mk[2] == 0.0f) continue;
-        float d[3], basis[16];
-        view_dir(pos, cams[v].pos, d);
-        sh_basis(d, basis);
+    const float* masks = reinterpret_cast<const float*>(gv + 3 * S);
+    for (int v0 = 0; v0 < nviews; v0 += G) {
+        bool seen[G];
+        float mk[G][3];
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch)
+        for (int k = 0; k < G; ++k) seen[k] = v0 + k < nviews && cnt[(size_t)(v0 + k) * n + i] != 0;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) shg[ch][k] += mk[ch] * basis[k];
+        for (int k = 0; k < G; ++k)
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) mk[k][ch] = seen[k] ? masks[ch * S + (size_t)(v0 + k) * n + i] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            if (mk[k][0] == 0.0f && mk[k][1] == 0.0f && mk[k][2] == 0.0f) continue;
+            float d[3], basis[16];
+            view_dir(pos, cams[v0 + k].pos, d);
+            sh_basis(d, basis);
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch)
+#pragma unroll
+                for (int q = 0; q < 16; ++q) shg[ch][q] += mk[k][ch] * basis[q];
+        }
     }
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) {
@@ -381,13 +398,25 @@ __global__ void __launch_bounds__(128, PART == 2 ? 8 : 6) k_geom_gauss(const flo
     if (PART == 1) return;
     // ---- geometry: sums over views
     float dpos[3] = {0.0f, 0.0f, 0.0f}, dop = 0.0f, dS[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, screen = 0.0f;
-    for (int v = 0; v < nviews; ++v) {
-        const size_t s = (size_t)v * n + i;
-        if (cnt[s] == 0) continue;
-        const float4 x0 = gv[s], x1 = gv[S + s], x2 = gv[2 * S + s];
-        dpos[0] += x0.x; dpos[1] += x0.y; dpos[2] += x0.z; dop += x0.w;
-        dS[0] += x1.x; dS[1] += x1.y; dS[2] += x1.z; dS[3] += x1.w;
-        dS[4] += x2.x; dS[5] += x2.y; screen += x2.z;
+    for (int v0 = 0; v0 < nviews; v0 += G) {
+        bool seen[G];
+        float4 x0[G], x1[G], x2[G];
+#pragma unroll
+        for (int k = 0; k < G; ++k) seen[k] = v0 + k < nviews && cnt[(size_t)(v0 + k) * n + i] != 0;
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            const size_t s = (size_t)(v0 + k) * n + i;
+            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            x0[k] = seen[k] ? gv[s] : z;
+            x1[k] = seen[k] ? gv[S + s] : z;
+            x2[k] = seen[k] ? gv[2 * S + s] : z;
+        }
+#pragma unroll
+        for (int k = 0; k < G; ++k) {  // an unseen view adds zeros
+            dpos[0] += x0[k].x; dpos[1] += x0[k].y; dpos[2] += x0[k].z; dop += x0[k].w;
+            dS[0] += x1[k].x; dS[1] += x1[k].y; dS[2] += x1[k].z; dS[3] += x1[k].w;
+            dS[4] += x2[k].x; dS[5] += x2[k].y; screen += x2[k].z;
+        }
     }
     const float4 p1 = params[(size_t)cap + i], p2 = params[2 * (size_t)cap + i];
     const float q[4] = {p1.x, p1.y, p1.z, p1.w};
@@ -481,8 +510,7 @@ __global__ void __launch_bounds__(128, 8) k_geom_sh(int n, int cap, const DevCam
     const AdamStep step = adam_step(a);
     const float4 p0 = a.params[i];
     const float pos[3] = {p0.x, p0.y, p0.z};
-    const float* mplane = reinterpret_cast<const float*>(gv + (ch == 0 ? 2 : 3) * S);
-    const int mlane = ch == 0 ? 3 : ch - 1;
+    const float* mask = reinterpret_cast<const float*>(gv + 3 * S) + ch * S;
     float shg[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) shg[k] = 0.0f;
@@ -492,7 +520,7 @@ __global__ void __launch_bounds__(128, 8) k_geom_sh(int n, int cap, const DevCam
 #pragma unroll
         for (int k = 0; k < VIEW_GROUP; ++k) c8[k] = v0 + k < nviews ? cnt[(size_t)(v0 + k) * n + i] : 0u;
 #pragma unroll
-        for (int k = 0; k < VIEW_GROUP; ++k) m8[k] = c8[k] ? mplane[((size_t)(v0 + k) * n + i) * 4 + mlane] : 0.0f;
+        for (int k = 0; k < VIEW_GROUP; ++k) m8[k] = c8[k] ? mask[(size_t)(v0 + k) * n + i] : 0.0f;
 #pragma unroll
         for (int k = 0; k < VIEW_GROUP; ++k) {
             if (m8[k] == 0.0f) continue;
@@ -524,7 +552,7 @@ void launch_geometry(const float4* params, int n, int cap, const DevCam* cams, i
     if (n <= 0) return;
     launch_geom_view(params, n, cap, cams, nviews, cnt, acc, rec, gcache, gv, st);
     AdamArgs a{};
-    k_geom_gauss<0><<<(n + 127) / 128, 128, 0, st>>>(params, n, cap, cams, nviews, cnt, gv, grads, accumulate, a);
+    (nviews > 2 ? k_geom_gauss<0, 0, 4> : k_geom_gauss<0, 0, 1>)<<<(n + 127) / 128, 128, 0, st>>>(params, n, cap, cams, nviews, cnt, gv, grads, accumulate, a);
 }
 
 void launch_geometry_adam(const DevCam* cams, int nviews, int n, int cap, const uint32_t* cnt, const float4* acc, const float4* rec,
@@ -532,7 +560,7 @@ void launch_geometry_adam(const DevCam* cams, int nviews, int n, int cap, const 
     if (n <= 0) return;
     launch_geom_view(a.params, n, cap, cams, nviews, cnt, acc, rec, gcache, gv, st);
     k_geom_sh<<<dim3((unsigned)((n + 127) / 128), 3), 128, 0, st>>>(n, cap, cams, nviews, cnt, gv, a);
-    k_geom_gauss<1, 2><<<(n + 127) / 128, 128, 0, st>>>(nullptr, n, cap, cams, nviews, cnt, gv, nullptr, 0, a);
+    (nviews > 2 ? k_geom_gauss<1, 2, 4> : k_geom_gauss<1, 2, 1>)<<<(n + 127) / 128, 128, 0, st>>>(nullptr, n, cap, cams, nviews, cnt, gv, nullptr, 0, a);
 }
 
 __global__ void __launch_bounds__(256) k_adam(int n, int cap, const float4* __restrict__ grads, AdamArgs a) {
