@@ -728,15 +728,16 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         if not args.no_rows and world == 1:
             line["next_rows"] = measure_next_rows(R, g, cfg.cameras[0], local_rank, cpu=not args.no_cpu_baseline)
         # kernels launched per batched step (+ memsets): term cache + project 2;
-        # compaction 3 (counts, scan, gather); depth sort 4 passes x 3; two
-        # count scans 2 x 2; emit 1; supertile sort 3 per 8 bits of the
-        # supertile id; tile lists 3 (masks, scan, writer); forward 1; loss 2;
+        # compaction 3 (counts, scan, gather); depth sort 4 passes x 3, or one for
+        # up to 65536 slots; entry scan 2, emit 1; supertile sort 3 per 8 bits of
+        # the supertile id; tile lists 3 (counts, scan, writer); forward 1; loss 2;
         # backward 1; geometry + Adam 3 (per view, SH half, geometry half)
         ltw, lth = (int(x) for x in layout[0].split("x"))
         cdiv = lambda a, b: -(-a // b)
         st_view = max(cdiv(cdiv(c.width, ltw), 4) * cdiv(cdiv(c.height, lth), 4) for c in cfg.cameras)
         st_bits = max(1, int(np.ceil(np.log2(max(2, V * st_view)))))
-        per_step = 2 + 3 + 12 + 4 + 1 + 3 * ((st_bits + 7) // 8) + 3 + 1 + 2 + 1 + 3
+        depth = 12 if V * n > 65536 else 1
+        per_step = 2 + 3 + depth + 2 + 1 + 3 * ((st_bits + 7) // 8) + 3 + 1 + 2 + 1 + 3
         line["gpu_launches"] = per_step * args.steps
         print(json.dumps(line), flush=True)
     if dist is not None:

@@ -469,7 +469,7 @@ int read_scalars(rgs_ctx* ctx) {
 // Only valid with a zero background, where a pixel whose reference tile list
 // is empty renders the same 0 as one whose splats all miss it.
 int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tiles, bool host_count, Binned& out,
-              bool project, bool prune, size_t st_cap = 0) {
+              bool project, bool prune, size_t st_cap = 0, float4* acc = nullptr) {
     // supertiles the buffers and scans cover: the batch's own unless the
     // caller (a captured graph replayed for other views) gives a bound
     if (!st_cap) st_cap = std::max<size_t>(ctx->hdr_h->total_st, 1);
@@ -480,7 +480,7 @@ int bin_batch(rgs_ctx* ctx, Scene& s, const DevCam* cams_dev, int V, size_t tile
     if (project)
         launch_project(s.params.as<float4>(), s.n, s.cap, cams_dev, V, ctx->opt.tile_w, ctx->opt.tile_h,
                        ctx->rec.as<float4>(), ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), prune ? 1 : 0,
-                       ctx->gcache.as<float4>(), ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), st);
+                       ctx->gcache.as<float4>(), ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), acc, st);
     mark(ctx, 1);
     // only the slots with tile pairs go through the depth sort, gathered in
     // slot order (the stable sort then still breaks depth ties by index)
@@ -659,7 +659,8 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
     if ((rc = ensure_gcache(ctx, s))) return rc;
     mark(ctx, 0);
     Binned b;
-    if ((rc = bin_batch(ctx, s, cams_dev, 1, tiles, true, b, true, zero_bg(bg)))) return rc;
+    if ((rc = bin_batch(ctx, s, cams_dev, 1, tiles, true, b, true, zero_bg(bg), 0, do_backward ? ctx->acc.as<float4>() : nullptr)))
+        return rc;
     BlendArgs fa = blend_args(ctx, s, cams_dev, 1, nullptr, tiles, b, bg, true);
     fa.bg_start = bg_start ? 1 : 0;
     if (study) {
@@ -690,7 +691,6 @@ int run_view_plain(rgs_ctx* ctx, Scene& s, const DevCam& dc_in, const float* tar
     CK(launch_loss(cams_dev, 1, (int)lb, ctx->rgb.as<float>(), lambda, ctx->dl.as<float>(), ctx->partials.as<float>(),
                    losses_dev, nullptr, ctx->opt.exact_loss != 0, st));
     mark(ctx, 7);
-    CK(cudaMemsetAsync(ctx->acc.p, 0, std::max<size_t>(s.n, 1) * 3 * sizeof(float4), st));
     BlendArgs ba = blend_args(ctx, s, cams_dev, 1, nullptr, tiles, b, bg, false);
     if (study) {
         ba.tstore = fa.tstore;
@@ -1488,7 +1488,7 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
     cudaMemcpyAsync(ctx->hdr.p, ctx->hdr_h, sizeof(StepHdr), cudaMemcpyHostToDevice, st);
     mark(ctx, 0);
     Binned b;
-    int rc = bin_batch(ctx, s, cams_dev, V, tiles_cap, false, b, true, zero_bg(bg), st_cap);
+    int rc = bin_batch(ctx, s, cams_dev, V, tiles_cap, false, b, true, zero_bg(bg), st_cap, ctx->acc.as<float4>());
     if (!rc) {
         BlendArgs fa = blend_args(ctx, s, cams_dev, V, &hd->total_tiles, tiles_cap, b, bg, true);
         launch_blend_forward(fa, ctx->opt.tile_w, ctx->opt.tile_h, st);
@@ -1501,7 +1501,6 @@ int capture_batched(rgs_ctx* ctx, int V, size_t tiles_cap, const float bg[3], fl
                                      ctx->opt.exact_loss != 0, st);
         if (le != cudaSuccess) rc = cuda_fail(ctx, le, "loss kernel launch");
         mark(ctx, 7);
-        cudaMemsetAsync(ctx->acc.p, 0, std::max<size_t>(S, 1) * 3 * sizeof(float4), st);
         BlendArgs ba = blend_args(ctx, s, cams_dev, V, &hd->total_tiles, tiles_cap, b, bg, false);
         launch_blend_backward(ba, ctx->opt.tile_w, ctx->opt.tile_h, st);
         mark(ctx, 8);
@@ -1582,7 +1581,7 @@ int batched_step(rgs_ctx* ctx, const uint32_t* views, int V, const float bg[3], 
         CK(cudaMemcpyAsync(ctx->hdr.p, ctx->hdr_h, sizeof(StepHdr), cudaMemcpyHostToDevice, ctx->st));
         launch_project(s.params.as<float4>(), s.n, s.cap, cams_dev, V, ctx->opt.tile_w, ctx->opt.tile_h, ctx->rec.as<float4>(),
                        ctx->cnt.as<uint32_t>(), ctx->dkey.as<uint32_t>(), zero_bg(bg) ? 1 : 0, ctx->gcache.as<float4>(),
-                       ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), ctx->st);
+                       ctx->spans.as<uint4>(), ctx->st_cnt.as<uint32_t>(), nullptr, ctx->st);
         launch_view_pairs(ctx->cnt.as<uint32_t>(), (uint32_t)s.n, V, ctx->view_pairs.as<unsigned long long>(), ctx->st);
         CK(cudaGetLastError());
         unsigned long long per[MAX_VIEWS], total = 0;

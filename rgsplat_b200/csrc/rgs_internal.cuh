@@ -185,11 +185,13 @@ void launch_check_finite(const float4* planes, int n, int cap, int* flag, cudaSt
 //       rectangle meets, or with prune, per supertile row, those from the first
 //       to the last that its kept spans meet.
 // st_cnt[s] = the entries again (their scan gathers four bytes a slot).
+// acc: where given, the three planes of gradient sums of the slots that are not
+// culled are zeroed (a backward pass follows; no other slot's are read).
 constexpr int SPAN_ROWS = 16;
 constexpr uint32_t SPANS_NONE = 0xffffffffu;
 void launch_project(const float4* params, int n, int cap, const DevCam* cams, int nviews,
                     int tile_w, int tile_h, float4* rec, uint32_t* cnt, uint32_t* dkey, int prune, float4* gcache,
-                    uint4* spans, uint32_t* st_cnt, cudaStream_t st);
+                    uint4* spans, uint32_t* st_cnt, float4* acc, cudaStream_t st);
 // Per-Gaussian view-independent projection terms ([2][cap] float4: opacity
 // and the 3D covariance's six entries), computed by launch_project first and
 // read by the geometry of the same step.
