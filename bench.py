@@ -232,10 +232,9 @@ def profiled_traffic(kernel_file: str):
 
 
 def profiled_issue_active(kernel: str):
-    """Fraction of issue slots the packed blend kernel kept busy, from the
-    committed ncu pipe-mix table (quarter-size capture of the same launch
-    shape; columns: forward scalar, forward packed, backward scalar, backward
-    packed)."""
+    """Fraction of issue slots the blend kernel kept busy, from the committed ncu
+    pipe-mix table (quarter-size capture of the same launch shape; columns:
+    forward before, forward now, backward before, backward now)."""
     col = {"k_blend_fwd": 3, "k_blend_bwd": 5}.get(kernel)
     try:
         for line in open(os.path.join(ROOT, "profiles", "blend_pipes_250k_8views.md")):

@@ -5,7 +5,8 @@
 // the result deterministic: inputs arrive in slot order, so equal keys keep
 // index order, which is the (tile, depth bits, index) order the oracle uses.
 //
-// Each pass is reduce-then-scan with a fixed grid (no inter-block waiting):
+// Up to 65536 pairs: all passes in one cluster launch (k_sort_cluster, below).
+// More: each pass is reduce-then-scan with a fixed grid (no inter-block waiting):
 // every block owns one contiguous chunk of the input.
 //   upsweep:   per-block digit histogram of its chunk          -> hist[b][d]
 //   scan:      one block turns hist into global offsets (digit-major order)
