@@ -60,7 +60,13 @@ void make_block(Pool& p) {
     if (m == MAP_FAILED) return;
     char* q = (char*)(((uintptr_t)m + HC_HUGE - 1) & ~(uintptr_t)(HC_HUGE - 1));
     madvise(q, HC_BLOCK, MADV_HUGEPAGE);  // a hint: small pages do the same, slower
-    if (cudaHostRegister(q, HC_BLOCK, cudaHostRegisterPortable) != cudaSuccess) {
+    // another thread of the program may be capturing a graph in a mode that would
+    // refuse this call
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaHostRegister(q, HC_BLOCK, cudaHostRegisterPortable);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
         cudaGetLastError();
         munmap(m, HC_BLOCK + HC_HUGE);
         return;

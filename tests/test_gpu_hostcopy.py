@@ -1,7 +1,8 @@
 """Large host copies (several threads through page-locked slabs) return what the
 small ones do: sizes on both sides of the 8 MiB threshold and of the 1 MiB chunk,
 into fresh and used arrays, from several threads with a context each, and again
-after the last context has given the slabs back."""
+after the last context has given the slabs back. The slabs exist from the first
+32 MiB of large copies on, which the first test brings about."""
 import threading
 
 import numpy as np
@@ -27,9 +28,16 @@ def _round_trip(n, seed):
     tr.ctx.close()
 
 
+def test_before_and_after_the_slabs_exist():
+    for n in (35_545, 150_000, 35_545, 400_001):
+        _round_trip(n, n)
+
+
 @pytest.mark.parametrize("n", [35_544, 35_545, 39_988, 39_989, 100_003, 400_001])
 def test_round_trip(n):
+    big = R.Trainer(np.zeros((150_000, 59), np.float32), [CAM])  # 35 MB: the slabs exist
     _round_trip(n, n)
+    big.ctx.close()
 
 
 def test_threads_with_a_context_each():
