@@ -24,8 +24,9 @@
 //     mask of the ones it can reach;
 //   * backward warps skip splats past the warp's largest last_contrib.
 // Backward gathers each warp's partial gradients of eight splats in shared
-// memory, reads them back transposed (four lanes per splat) and issues one
-// 3 x 16-byte vector reduction (red.global.add.v4.f32) per splat per warp.
+// memory, reads them back transposed (four lanes per splat) and adds 48 bytes per
+// splat and warp to global memory: colour and opacity as one red.v4.f32, the
+// conic's three sums in 64 bits, the mean as a red.v2.f32.
 //
 // CTA tiles other than 16x16 keep the reference's per-pixel semantics: each
 // record carries its reference-tile rectangle in pixels and a pixel only
@@ -319,6 +320,14 @@ __device__ __forceinline__ void red_add_v4(float4* addr, float x, float y, float
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
+__device__ __forceinline__ void red_add_v2(float2* addr, float x, float y) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(addr), "f"(x), "f"(y) : "memory");
+}
+
+__device__ __forceinline__ void red_add_f64(double* addr, double x) {
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(addr), "d"(x) : "memory");
+}
+
 // One pixel of the backward decided with the forward's own arithmetic: nal is
 // minus its alpha (0 when it does not take the splat) and um minus the raw
 // alpha that scales dL/dalpha (0 when the raw alpha was clamped,
@@ -364,8 +373,13 @@ __device__ __noinline__ float2 bwd_exact_pixel(float dx, float dy, float4 q, flo
 // column sums (colour x3, u, u dy, u dy^2 with u = dL/dpower) for up to
 // BWD_GRP splats in the warp's own shared memory, then the warp reads them
 // transposed, four lanes per splat, each adding eight columns, expands the
-// moments in dx, and issues one red.global.add.v4 per accumulator plane. The
-// stores and loads are swizzled by the splat's place in the group, so neither
+// moments in dx, and adds them to the slot's sums with three reductions. Those of
+// the conic are 64-bit: across tiles they add up in any order, and the geometry's
+// gradient is a difference of them that cancels by the covariance's condition
+// number; in 32 bits, two passes over a scene of needles differed by the whole of
+// their rotations' gradient, and over 3M anisotropic Gaussians by 1 to 5 % of all
+// gradients (now 5e-7; the same time, 6.18 ms a step of 1M x 8 views and 31.7 of
+// 3M). The stores and loads are swizzled by the splat's place in the group, so neither
 // has bank conflicts. Warps share only the staged batch and the two barriers
 // around it.
 //
@@ -526,9 +540,14 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(B
                 }
                 // the sums are of negated terms
                 if (g < cnt) {
+                    // a slot's second and third record: conic a, b | conic c, (sx, sy)
+                    double* conic = reinterpret_cast<double*>(a.acc + (q == 3 ? 2 * S : S) + slot) + (q == 2 ? 1 : 0);
+                    const float part = q == 1 ? 0.5f * u2 : q == 2 ? w1 : 0.5f * w2;
                     if (q == 0) red_add_v4(a.acc + slot, -c0, -c1, -c2, -u0 / ctr.z);
-                    if (q == 1) red_add_v4(a.acc + S + slot, 0.5f * u2, w1, 0.5f * w2, -__fmaf_rn(cq.y, w0, cq.x * u1));
-                    if (q == 2) red_add_v4(a.acc + 2 * S + slot, -__fmaf_rn(cq.z, w0, cq.y * u1), 0.0f, 0.0f, 0.0f);
+                    else red_add_f64(conic, (double)part);
+                    if (q == 3)
+                        red_add_v2(reinterpret_cast<float2*>(a.acc + 2 * S + slot) + 1, -__fmaf_rn(cq.y, w0, cq.x * u1),
+                                   -__fmaf_rn(cq.z, w0, cq.y * u1));
                 }
                 __syncwarp();
                 cnt = 0;

@@ -2274,9 +2274,12 @@ int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs
         CK(cudaMemcpyAsync(acc.data(), ctx->acc.p, 3 * n * sizeof(float4), cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
         for (size_t i = 0; i < n; ++i) {
-            float4 a = acc[i], c = acc[n + i], d = acc[2 * n + i];
+            const float4 a = acc[i];
+            const BlendSums b = blend_sums(acc.data(), n, i);
             float* o = acc9 + i * 9;
-            o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = c.x; o[5] = c.y; o[6] = c.z; o[7] = c.w; o[8] = d.x;
+            o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+            for (int k = 0; k < 3; ++k) o[4 + k] = (float)b.conic[k];
+            o[7] = b.mean[0]; o[8] = b.mean[1];
         }
     }
     if (dl_dpix) {

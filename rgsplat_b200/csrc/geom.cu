@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__
     const size_t s = (size_t)v * n + i;
     if (cnt[s] == 0) return;
     const DevCam& c = cams[v];
-    const float4 a0 = acc[s], a1 = acc[S + s], a2 = acc[2 * S + s];
+    const float4 a0 = acc[s];
+    const BlendSums sums = blend_sums(acc, S, s);
     const float4 col = rec[2 * S + s];
     const float4 p0 = params[i];
     const float pos[3] = {p0.x, p0.y, p0.z};
@@ -112,13 +113,17 @@ __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__
         b2d = s2.m[0][1];
         c2d = s2.m[1][1] + 0.3f;
     }
-    // conic -> 2D covariance (backward.rs:546-554)
-    const float ga = a1.x, gb = a1.y, gc = a1.z;
+    // conic -> 2D covariance (backward.rs:546-554); the three terms of each cancel by
+    // the covariance's condition number, so they are formed in 64 bits
     const float det = a2d * c2d - b2d * b2d;
     const float idet2 = 1.0f / (det * det);
-    const float dl_da = (-ga * c2d * c2d + gb * b2d * c2d - gc * b2d * b2d) * idet2;
-    const float dl_db = (2.0f * ga * b2d * c2d - gb * (det + 2.0f * b2d * b2d) + 2.0f * gc * a2d * b2d) * idet2;
-    const float dl_dc = (-ga * b2d * b2d + gb * a2d * b2d - gc * a2d * a2d) * idet2;
+    float dl_da, dl_db, dl_dc;
+    {
+        const double ga = sums.conic[0], gb = sums.conic[1], gc = sums.conic[2], a = a2d, b = b2d, c = c2d;
+        dl_da = (float)((gb * b - ga * c) * c - gc * b * b) * idet2;
+        dl_db = (float)(2.0 * b * (ga * c + gc * a) - gb * ((double)det + 2.0 * b * b)) * idet2;
+        dl_dc = (float)((gb * b - gc * a) * a - ga * b * b) * idet2;
+    }
     // T = J W, rows u0, u1 (row 2 of J is zero) (backward.rs:556-564)
     const float itz = 1.0f / tz, itz2 = itz * itz, itz3 = itz2 * itz;
     const float j00 = fx * itz, j02 = -fx * tx * itz2, j11 = fy * itz, j12 = -fy * ty * itz2;
@@ -144,7 +149,7 @@ __global__ void __launch_bounds__(128, 8) k_geom_view(const float4* __restrict__
     dS[4] = u0[1] * r0[2] + u1[1] * r1[2];
     dS[5] = u0[2] * r0[2] + u1[2] * r1[2];
     // mean through (sx, sy) and through J(pcam) (backward.rs:578-605)
-    const float asx = a1.w, asy = a2.x;
+    const float asx = sums.mean[0], asy = sums.mean[1];
     float dp[3] = {asx * j00, asy * j11, asx * j02 + asy * j12};
     {
         // Sigma u0, Sigma u1, Sigma w2 with w2 = row 2 of W

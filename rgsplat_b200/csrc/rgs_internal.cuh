@@ -16,8 +16,9 @@
 //                          (conic a, b, c, pixel rect x0|x1<<16),
 //                          (r, g, b, pixel rect y0|y1<<16)
 //   cnt     [S] u32        number of CTA tiles the splat touches (0 = culled)
-//   acc     [3][S] float4  blend-backward accumulators (color3, opacity,
-//                          conic3, sx, sy) of backward.rs:92-99
+//   acc     [3][S] 16 B    blend-backward accumulators of backward.rs:92-99:
+//                          color3, opacity | conic a, b in f64 | conic c in
+//                          f64, sx, sy (blend_sums)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -277,6 +278,27 @@ size_t supertile_chunks(size_t entries);
 // Per entry the 16-tile mask, the per-chunk counts and their scans, then the
 // tile lists and the ranges of every tile that some entry's supertile holds.
 void launch_supertile_lists(const SupertileArgs& a, cudaStream_t st);
+
+// What the blend backward summed of slot s for its conic and screen position.
+// The conic's sums are in 64 bits: the covariance's gradient is a difference of
+// them that cancels by the covariance's condition number (10^6 for a Gaussian
+// hundreds of pixels long and half a pixel wide), so that 32-bit sums left it a
+// rounding of the order the tiles happened to add in.
+struct BlendSums {
+    double conic[3];
+    float mean[2];
+};
+__host__ __device__ inline BlendSums blend_sums(const float4* acc, size_t S, size_t s) {
+    const double2 ab = *reinterpret_cast<const double2*>(acc + S + s);
+    BlendSums r;
+    r.conic[0] = ab.x;
+    r.conic[1] = ab.y;
+    r.conic[2] = *reinterpret_cast<const double*>(acc + 2 * S + s);
+    const float2 m = reinterpret_cast<const float2*>(acc + 2 * S + s)[1];
+    r.mean[0] = m.x;
+    r.mean[1] = m.y;
+    return r;
+}
 
 // blend.cu
 struct BlendArgs {
