@@ -55,17 +55,23 @@ Pool& pool() {
     return *p;
 }
 
+// Another thread of the program may be capturing a graph in a mode that would refuse
+// this thread's call outside the relaxed mode.
+template <class Call>
+cudaError_t relaxed(const Call& call) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = call();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
 void make_block(Pool& p) {
     void* m = mmap(nullptr, HC_BLOCK + HC_HUGE, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
     if (m == MAP_FAILED) return;
     char* q = (char*)(((uintptr_t)m + HC_HUGE - 1) & ~(uintptr_t)(HC_HUGE - 1));
     madvise(q, HC_BLOCK, MADV_HUGEPAGE);  // a hint: small pages do the same, slower
-    // another thread of the program may be capturing a graph in a mode that would
-    // refuse this call
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaHostRegister(q, HC_BLOCK, cudaHostRegisterPortable);
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = relaxed([&] { return cudaHostRegister(q, HC_BLOCK, cudaHostRegisterPortable); });
     if (e != cudaSuccess) {
         cudaGetLastError();
         munmap(m, HC_BLOCK + HC_HUGE);
@@ -77,11 +83,16 @@ void make_block(Pool& p) {
     p.idle_n = HC_SLABS;
 }
 
-// With no context left and every slab back.
+// With no context left and every slab back. A block that the driver does not let go
+// stays mapped, for the next context: its addresses must not become another array's
+// while they are taken for page-locked.
 void free_block(Pool& p) {
     if (p.users != 0 || p.idle_n != (p.block ? HC_SLABS : 0)) return;
     if (p.block) {
-        cudaHostUnregister(p.block);
+        if (relaxed([&] { return cudaHostUnregister(p.block); }) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
         munmap(p.map, HC_BLOCK + HC_HUGE);
     }
     p.map = nullptr;

@@ -3,6 +3,8 @@
 // when something waits for them, and cudaStreamPerThread names another queue in
 // every thread.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cstring>
 #include <deque>
@@ -30,6 +32,9 @@ std::recursive_mutex mu;
 std::map<Key, Queue> queues;
 std::map<char*, size_t> registered;
 int fail_after = -1;  // the copies that still succeed (-1: all)
+bool capturing = false;       // another thread captures a graph in the global mode
+bool no_unregister = false;  // cudaHostUnregister fails whatever the mode
+thread_local cudaStreamCaptureMode capture_mode = cudaStreamCaptureModeGlobal;
 
 Queue& queue_of(cudaStream_t st) {
     return queues[{st, st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id()}];
@@ -61,8 +66,7 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* mode) {
-    thread_local cudaStreamCaptureMode mine = cudaStreamCaptureModeGlobal;
-    std::swap(mine, *mode);
+    std::swap(capture_mode, *mode);
     return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
@@ -73,11 +77,14 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
 }
 cudaError_t cudaHostRegister(void* p, size_t n, unsigned) {
     std::lock_guard<std::recursive_mutex> lock(mu);
+    if (capturing && capture_mode != cudaStreamCaptureModeRelaxed) return cudaErrorStreamCaptureUnsupported;
     registered[(char*)p] = n;
     return cudaSuccess;
 }
 cudaError_t cudaHostUnregister(void* p) {
     std::lock_guard<std::recursive_mutex> lock(mu);
+    if (no_unregister) return cudaErrorUnknown;
+    if (capturing && capture_mode != cudaStreamCaptureModeRelaxed) return cudaErrorStreamCaptureUnsupported;
     registered.erase((char*)p);
     return cudaSuccess;
 }
@@ -144,4 +151,17 @@ int fake_failing(size_t bytes, int good, int to_host) {
 }
 
 int fake_registered() { return (int)registered.size(); }
+void fake_capturing(int on) { capturing = on != 0; }
+void fake_no_unregister(int on) { no_unregister = on != 0; }
+
+// Registered ranges that are no longer mapped, which no program may leave behind.
+int fake_dangling() {
+    int bad = 0;
+    for (auto& r : registered) {
+        const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+        std::vector<unsigned char> in((r.second + page - 1) / page);
+        bad += mincore((void*)((uintptr_t)r.first & ~(page - 1)), r.second, in.data()) != 0;
+    }
+    return bad;
+}
 }

@@ -44,3 +44,31 @@ def test_order_of_the_callers_stream(lib, nbytes, per_thread):
 def test_error(lib, good, to_host):
     assert lib.fake_failing(40 * MIB, good, to_host) == 0
     assert lib.fake_ordered(20 * MIB, 0) == 0
+
+
+def test_last_context_goes_during_a_capture(lib):
+    """Another thread's capture in the global mode refuses cudaHostUnregister to a
+    thread that is not in the relaxed mode; the block is given back all the same."""
+    lib.fake_capturing(1)
+    lib.fake_user(-1)
+    lib.fake_capturing(0)
+    assert lib.fake_dangling() == 0
+    assert lib.fake_registered() == 0
+    lib.fake_user(1)
+    assert lib.fake_ordered(32 * MIB, 0) == 0
+    assert lib.fake_registered() == 1
+
+
+def test_block_that_cannot_be_unregistered(lib):
+    """What the driver still holds as page-locked stays mapped, and is used again."""
+    lib.fake_no_unregister(1)
+    lib.fake_user(-1)
+    assert lib.fake_dangling() == 0
+    lib.fake_user(1)
+    assert lib.fake_ordered(40 * MIB, 0) == 0
+    lib.fake_no_unregister(0)
+    lib.fake_user(-1)
+    assert lib.fake_registered() == 0
+    lib.fake_user(1)
+    assert lib.fake_ordered(32 * MIB, 0) == 0
+    assert lib.fake_registered() == 1
