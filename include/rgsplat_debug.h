@@ -59,6 +59,14 @@ int rgs_debug_backward(rgs_ctx* ctx, const float* gaussians, size_t n, const rgs
  * wherever the two evaluations could disagree.) */
 int rgs_debug_exp_sfu_error(rgs_ctx* ctx, float lo, float hi, uint32_t n, float* max_rel);
 
+/* The backward blend's own alpha against 64 bits over n x n powers on [power_lo, 0]
+ * (power_lo >= -8) and opacities on [opacity_lo, opacity_hi] (within [1/255, 1]):
+ * alpha_rel, its largest relative error; decision, the largest error (in log2 units)
+ * of the value that decides alpha >= 1/255 without the forward's arithmetic, near
+ * that decision. */
+int rgs_debug_backward_alpha_error(rgs_ctx* ctx, float power_lo, float opacity_lo, float opacity_hi, uint32_t n,
+                                   float* alpha_rel, float* decision);
+
 /* Pixels of the view at position k of the trainer's most recent batched pass
  * (rgs_trainer_step or rgs_trainer_backward with RGS_STEP_BATCHED that ran as
  * one view group), read from the batch's own buffers: rgb w*h*3, final T w*h

@@ -356,17 +356,19 @@ __device__ __noinline__ float2 bwd_exact_pixel(float dx, float dy, float4 q, flo
 // views, 1.57 -> 0.57 ms on 97k x 3 views of 1277x719 with a white background,
 // 262 -> 52 us on 10k at 256x256 (where one tile's serial walk is the time).
 //
-// Alpha comes from one SFU exponential of p = power log2(e) + log2(opacity),
-// with the power rounded exactly as the forward rounds it. (A power from two
+// Alpha is the opacity times one SFU exponential of t = power log2(e), with the
+// power rounded exactly as the forward rounds it. (A power from two
 // packed FMAs over prescaled coefficients saves four packed instructions per
 // pixel pair and ran 4 % faster; but an ill-conditioned conic's terms cancel,
-// and its alpha then strays from the forward's by up to 1e-4.) The
-// contributing set must be the forward's exactly, so a pixel whose p lies
-// within BWD_BAND of a decision (alpha >= 1/255; alpha_raw > 0.99; power > 0,
-// where p reaches log2(opacity)) is decided by bwd_exact_pixel: the roundings
-// of p (|p| <= 8), of log2(opacity) and of the forward's own alpha add up to
-// less than 2e-6 in log2 units, half the band. Every test reads a NaN as
-// "decide exactly".
+// and its alpha then strays from the forward's by up to 1e-4. The opacity as
+// log2(opacity) in the exponent saves one; but its rounding, up to 3e-7 of
+// alpha, is then every pixel's.) The
+// contributing set must be the forward's exactly, so a pixel whose t lies
+// within BWD_BAND of a decision (alpha >= 1/255; alpha_raw > 0.99; power > 0)
+// is decided by bwd_exact_pixel: the roundings of t (|t| <= 8), of the limits
+// and of the forward's own alpha add up to less than 2e-6 in log2 units, half
+// the band. A NaN conic, colour or opacity makes the limit NaN, and every pixel
+// of that splat is decided exactly.
 //
 // The nine gradient sums of a splat are not reduced across the warp per splat
 // (14 shuffles and two shared atomics each, serialised): a lane stores its six
@@ -393,16 +395,24 @@ __device__ __noinline__ float2 bwd_exact_pixel(float dx, float dy, float4 q, flo
 constexpr float BWD_BAND = 4e-6f;
 constexpr int BWD_GRP = 8;
 
+// A splat's limits on t: it contributes where t + reach > 0; up to `limit` its raw
+// alpha is at most 0.99 and its power at most 0.
+struct BwdLimits {
+    float reach, limit;
+};
+__device__ __forceinline__ BwdLimits bwd_limits(float opacity) {
+    const float lop = log2f(opacity);
+    return {7.99435344f + lop, fminf(-0.0144995697f - lop, lop != lop ? lop : 0.0f) - BWD_BAND};  // log2(255), log2(0.99)
+}
+constexpr float BWD_T = -0.5f * 1.44269504f;  // t of -2 power
+
 template <int TW, int TH, bool RECT, int PPT, bool STORE = false>
 __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(BlendArgs a) {
     constexpr int NT = TW * TH / PPT;
     constexpr int NW = NT / 32;
     constexpr int H = PPT / 2;
-    constexpr float LOG2E = 1.44269504f;
-    constexpr float L255 = 7.99435344f;    // log2(255)
-    constexpr float L099 = -0.0144995697f;  // log2(0.99)
-    __shared__ float4 s_a2[2][NT];  // sx, sy, opacity, log2(opacity)
-    __shared__ float4 s_c2[2][NT];  // a, b, c, largest p decided without the exact arithmetic
+    __shared__ float4 s_a2[2][NT];  // sx, sy, -opacity, reach
+    __shared__ float4 s_c2[2][NT];  // a, b, c, limit
     __shared__ float4 s_k2[2][NT];  // colour, power floor
     __shared__ uint2 s_r[RECT ? NT : 1];
     __shared__ uint32_t s_slot[NT];
@@ -489,9 +499,10 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(B
                 const float4 A = s_a[tid], Q = s_c[tid], K = s_k[tid];
                 const float thr = power_floor(A.z);
                 wm = reached_warps<NW, RW>(A, Q, thr, x0c, x1c, ty * TH, c.height);
-                const float lop = log2f(A.z);
-                s_a[tid].w = lop;
-                s_c[tid].w = not_sane(Q, K) ? __int_as_float(0x7fc00000) : fminf(L099, lop) - BWD_BAND;
+                const BwdLimits lim = bwd_limits(A.z);
+                s_a[tid].z = -A.z;
+                s_a[tid].w = lim.reach;
+                s_c[tid].w = not_sane(Q, K) ? __int_as_float(0x7fc00000) : lim.limit;
                 s_k[tid].w = thr;
                 s_slot[tid] = here;
                 if (RECT) s_r[tid] = make_uint2(__float_as_uint(Q.w), __float_as_uint(K.w));
@@ -543,7 +554,7 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(B
                     // a slot's second and third record: conic a, b | conic c, (sx, sy)
                     double* conic = reinterpret_cast<double*>(a.acc + (q == 3 ? 2 * S : S) + slot) + (q == 2 ? 1 : 0);
                     const float part = q == 1 ? 0.5f * u2 : q == 2 ? w1 : 0.5f * w2;
-                    if (q == 0) red_add_v4(a.acc + slot, -c0, -c1, -c2, -u0 / ctr.z);
+                    if (q == 0) red_add_v4(a.acc + slot, -c0, -c1, -c2, u0 / ctr.z);
                     else red_add_f64(conic, (double)part);
                     if (q == 3)
                         red_add_v2(reinterpret_cast<float2*>(a.acc + 2 * S + slot) + 1, -__fmaf_rn(cq.y, w0, cq.x * u1),
@@ -574,25 +585,25 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(B
                         // -2 power = (tdx + t2b dy) + (c dy) dy
                         const float2 s1 = __ffma2_rn(__fmul2_rn(bc2(t2b), dy[h]), one2, bc2(tdx));
                         const float2 s2 = __ffma2_rn(__fmul2_rn(__fmul2_rn(bc2(Q.z), dy[h]), dy[h]), one2, s1);
-                        const float2 p = __ffma2_rn(s2, bc2(-0.5f * LOG2E), bc2(A.w));
-                        const float2 d = __fadd2_rn(p, bc2(L255));
+                        const float2 t = __fmul2_rn(s2, bc2(BWD_T));
+                        const float2 d = __fadd2_rn(t, bc2(A.w));
                         bool a0 = li <= lc[2 * h], a1 = li <= lc[2 * h + 1];
                         if (RECT) {
                             const uint2 r = s_r[k];
                             a0 = a0 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h);
                             a1 = a1 && in_rect(__uint_as_float(r.x), __uint_as_float(r.y), px, py0 + 2 * h + 1);
                         }
-                        sure = sure && fminf(fabsf(d.x), fabsf(d.y)) >= BWD_BAND && fmaxf(p.x, p.y) <= Q.w;
+                        sure = sure && fminf(fabsf(d.x), fabsf(d.y)) >= BWD_BAND && fmaxf(t.x, t.y) <= Q.w;
                         a0 = a0 && d.x > 0.0f;
                         a1 = a1 && d.y > 0.0f;
                         any = any || a0 || a1;
-                        const float e0 = ex2_sfu(p.x), e1 = ex2_sfu(p.y);
-                        nal[h] = make_float2(a0 ? -e0 : 0.0f, a1 ? -e1 : 0.0f);
+                        const float2 e = __fmul2_rn(bc2(A.z), make_float2(ex2_sfu(t.x), ex2_sfu(t.y)));
+                        nal[h] = make_float2(a0 ? e.x : 0.0f, a1 ? e.y : 0.0f);
                         um[h] = nal[h];
                     }
                     float4 K = s_k[k];
                     if (!sure) {
-                        const float4 q = make_float4(Q.x, Q.y, Q.z, A.z);
+                        const float4 q = make_float4(Q.x, Q.y, Q.z, -A.z);
 #pragma unroll
                         for (int h = 0; h < H; ++h) {
                             const float2 zero = make_float2(0.0f, 0.0f);
@@ -771,6 +782,38 @@ __global__ void k_exp_sfu_error(float lo, float hi, uint32_t n, unsigned int* ou
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+}
+
+// The backward's alpha and its 1/255 decision against 64 bits, as float bits: out[0]
+// the largest relative error of alpha over n x n powers (evenly on [power_lo, 0])
+// and opacities (by ratio on [op_lo, op_hi]), out[1] the largest error of t + reach
+// over powers within 3e-5 of the decision.
+__global__ void k_bwd_alpha_error(float power_lo, float op_lo, float op_hi, uint32_t n, unsigned int* out) {
+    float m = 0.0f, d = 0.0f;
+    const float step = 1.0f / (float)(n > 1 ? n - 1 : 1);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n * n; i += gridDim.x * blockDim.x) {
+        const float op = op_lo * powf(op_hi / op_lo, (float)(i / n) * step);
+        const float power = power_lo * ((float)(i % n) * step);
+        const float al = op * ex2_sfu(-2.0f * power * BWD_T);
+        m = fmaxf(m, (float)fabs((double)al / ((double)op * exp((double)power)) - 1.0));
+        const float cut = -logf(255.0f * op) + ((float)(i % 61u) - 30.0f) * 1e-6f;
+        if (!(cut <= 0.0f)) continue;
+        const float reach = -2.0f * cut * BWD_T + bwd_limits(op).reach;
+        d = fmaxf(d, (float)fabs((double)reach - log2(255.0 * (double)op * exp((double)cut))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        d = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(out, __float_as_uint(m));
+        atomicMax(out + 1, __float_as_uint(d));
+    }
+}
+
+void launch_bwd_alpha_error(float power_lo, float op_lo, float op_hi, uint32_t n, unsigned int* out, cudaStream_t st) {
+    k_bwd_alpha_error<<<device_sm_count() * 4, 256, 0, st>>>(power_lo, op_lo, op_hi, n, out);
 }
 
 void launch_exp_sfu_error(float lo, float hi, uint32_t n, unsigned int* out, cudaStream_t st) {

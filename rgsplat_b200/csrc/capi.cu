@@ -2325,6 +2325,26 @@ int rgs_debug_exp_sfu_error(rgs_ctx* ctx, float lo, float hi, uint32_t n, float*
     return RGS_OK;
 }
 
+int rgs_debug_backward_alpha_error(rgs_ctx* ctx, float power_lo, float opacity_lo, float opacity_hi, uint32_t n, float* alpha_rel,
+                                   float* decision) {
+    int rc = check_ctx(ctx);
+    if (rc) return rc;
+    if (!alpha_rel || !decision || n == 0 || n > 16384 || !(power_lo >= -8.0f) || !(power_lo <= 0.0f) ||
+        !(opacity_lo >= 1.0f / 255.0f) || !(opacity_lo <= opacity_hi) || !(opacity_hi <= 1.0f))
+        return fail(ctx, RGS_ERR_INVALID_ARG, "need -8 <= power_lo <= 0, 1/255 <= opacity_lo <= opacity_hi <= 1, 0 < n <= 16384");
+    CK(ctx->view_pairs.ensure(MAX_VIEWS * 8));
+    unsigned int* out = ctx->view_pairs.as<unsigned int>();
+    float h[2] = {0.0f, 0.0f};
+    CK(cudaMemsetAsync(out, 0, 8, ctx->st));
+    launch_bwd_alpha_error(power_lo, opacity_lo, opacity_hi, n, out, ctx->st);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h, out, 8, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    *alpha_rel = h[0];
+    *decision = h[1];
+    return RGS_OK;
+}
+
 int rgs_debug_trainer_batch_pixels(rgs_ctx* ctx, size_t k, float* rgb, float* final_t, float* dl_dpix) {
     int rc = check_ctx(ctx);
     if (rc) return rc;

@@ -333,6 +333,9 @@ void launch_blend_store_all(const BlendArgs& a, bool fwd, cudaStream_t st);
 // Largest relative difference of the backward's SFU exponential from the
 // forward's exp over n points on [lo, hi] (float bits, atomicMax into *out).
 void launch_exp_sfu_error(float lo, float hi, uint32_t n, unsigned int* out, cudaStream_t st);
+// Largest errors of the backward's alpha (relative) and of its 1/255 decision
+// (base-2 exponent) against 64 bits, over n x n powers and opacities.
+void launch_bwd_alpha_error(float power_lo, float op_lo, float op_hi, uint32_t n, unsigned int* out, cudaStream_t st);
 // (pixel, splat) pairs the forward and backward blends of a pass evaluated,
 // from its final T, last contributors and tile ranges: out[0] forward,
 // out[1] backward (added to; u64).

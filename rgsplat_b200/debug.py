@@ -95,3 +95,14 @@ def exp_sfu_error(lo: float = -8.0, hi: float = 0.0, n: int = 1 << 24, ctx: Cont
     out = np.zeros(1, np.float32)
     ctx.check(ctx.lib.rgs_debug_exp_sfu_error(ctx.handle, float(lo), float(hi), int(n), _fp(out)))
     return float(out[0])
+
+
+def backward_alpha_error(power_lo: float, opacity_lo: float, opacity_hi: float, n: int = 2048,
+                         ctx: Context | None = None) -> tuple[float, float]:
+    """Largest errors of the backward blend's alpha (relative) and of its 1/255
+    decision (log2 units) against 64 bits over powers and opacities."""
+    ctx = ctx or default_context()
+    rel, dec = np.zeros(1, np.float32), np.zeros(1, np.float32)
+    ctx.check(ctx.lib.rgs_debug_backward_alpha_error(ctx.handle, float(power_lo), float(opacity_lo), float(opacity_hi), int(n),
+                                                     _fp(rel), _fp(dec)))
+    return float(rel[0]), float(dec[0])
