@@ -114,7 +114,11 @@ __device__ __forceinline__ bool not_sane(const float4& Q, const float4& K) {
 // bit mask of the staged splats that can reach its own strip of rows (about half
 // of the (strip, splat) pairs of a tile's list cannot), formed by one ballot per
 // 32 splats from the strip tests of the thread that staged each. A warp whose
-// pixels all pass by a splat asks whether any is still alive, else it is done.
+// pixels all pass by a splat asks whether any is still alive, else it is done; the
+// tile ends before the first batch that finds no pixel of it alive. (That vote on
+// the warps' own flags ended no tile with a strip below the image: an opaque scene at
+// 1600x1064, two thirds of a tile row, took 260 us, now 106. A warp that starts out
+// done where its strip is below the image cost all others 1 to 3 %.)
 //
 // Measured (1M Gaussians x 8 views): 1.80 ms for the loop that compacted each
 // batch by the tile test and visited every kept splat; 1.42 ms now. 97k x 3
@@ -177,7 +181,10 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 6 : 12) k_blend_fwd(
         fetch_entry(a, S, here, &s_a2[0][tid], &s_c2[0][tid], &s_k2[0][tid]);
         int buf = 0;
         for (uint32_t b0 = rg.x; b0 < rg.y; b0 += NT, buf ^= 1) {
-            if (__syncthreads_and(done)) break;
+            bool alive = false;
+#pragma unroll
+            for (int h = 0; h < H; ++h) alive = alive || !(T[h].x < 1e-4f) || !(T[h].y < 1e-4f);
+            if (__syncthreads_and(!alive)) break;
             fetch_entry(a, S, next, &s_a2[buf ^ 1][tid], &s_c2[buf ^ 1][tid], &s_k2[buf ^ 1][tid]);
             float4* s_a = s_a2[buf];
             float4* s_c = s_c2[buf];
@@ -619,7 +626,9 @@ __global__ void __launch_bounds__(TW * TH / PPT, PPT == 2 ? 5 : 9) k_blend_bwd(B
                             um[h] = make_float2(x0.y, x1.y);
                             any = any || x0.x != 0.0f || x1.x != 0.0f;
                         }
-                        // a colour that is not finite reaches no pixel that does not take it
+                        // a colour that is not finite reaches no thread whose pixels all pass
+                        // the splat by (the other pixels of a thread that takes it lie in the
+                        // loss window of a pixel that is NaN, and so is their dL/dpixel)
                         if (!any) K = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                     if (!__any_sync(0xffffffffu, any)) continue;
