@@ -246,28 +246,49 @@ __device__ __forceinline__ float adam_divide(float m1, float m2, float lr, const
     return lr * m1h / (sqrtf(m2h) + a.eps);
 }
 
-// The same without a branch, for values in a range that `ok` reports: quotients and
-// root are one hardware approximation and one correction by the exact remainder
-// each (Markstein, IBM J. Res. Dev. 34(1), 1990: the corrected value is the
-// rounded one, save for rare cases an ulp off). 0 <= m2; m2 = 0 has root 0.
-__device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, const AdamArgs& a, const AdamStep& s, bool& ok) {
-    float q = m1 * s.r1;
-    const float m1h = __fmaf_rn(__fmaf_rn(-q, s.bc1, m1), s.r1, q);
-    q = m2 * s.r2;
-    const float m2h = __fmaf_rn(__fmaf_rn(-q, s.bc2, m2), s.r2, q);
+// Rounded quotient a / b from the rounded reciprocal y of b > 0 (Markstein, IBM J.
+// Res. Dev. 34(1), 1990): the product, corrected by the exact remainder. The product
+// is off by less than half an ulp for y and half for itself, so near a tie it is one
+// of the tie's two neighbours and the correction rounds as the quotient does. a is 0
+// (and the quotient the same zero) or at least 2^-100, so that the remainder is exact.
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+    const float q = a * y;
+    return __fmaf_rn(-__fmaf_rn(q, b, -a), y, q);
+}
+
+// Whether values met so far are in the range of adam_divide_fast.
+struct AdamRange {
+    uint32_t least = 0xffffffffu;       // of 2 bits(x) - 1, x zero or at least 2^-100
+    uint32_t lo = 0xffffffffu, hi = 0;  // of the denominators' bits (hi: and of m2's, below 0 too large)
+    bool small = true;                  // every |update| <= 2^60
+    __device__ __forceinline__ void nonzero(float x) { least = min(least, 2u * __float_as_uint(x) - 1u); }
+    __device__ __forceinline__ bool all() const {
+        return small && least >= 2u * (27u << 23) - 1u && lo >= 67u << 23 && hi <= 147u << 23;  // 2^-100, 2^-60, 2^20
+    }
+};
+
+// The same update without a branch and with the same roundings, for values in a
+// range that `range` reports. The denominator's reciprocal and the root are one
+// hardware approximation and one such correction each; both were compared with the
+// rounded values over every mantissa (the root over every float of [2^-100, 2^40]),
+// and the quotients over 2^33 pairs, 9 10^7 of the nearest to a tie among them: none
+// differs. 0 <= m2, and m2 = 0 has root 0.
+__device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, const AdamArgs& a, const AdamStep& s, AdamRange& range) {
+    const float m1h = quotient(m1, s.bc1, s.r1), m2h = quotient(m2, s.bc2, s.r2);
     float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(m2h));
-    q = m2h * y;
-    float root = __fmaf_rn(__fmaf_rn(-q, q, m2h), 0.5f * y, q);
-    const bool none = m2h == 0.0f;
-    root = none ? 0.0f : root;
-    const float num = lr * m1h, den = root + a.eps;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(m2h, 0x1p-100f)));
+    float q = m2h * y;
+    const float num = lr * m1h, den = __fmaf_rn(__fmaf_rn(-q, q, m2h), 0.5f * y, q) + a.eps;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den));
     y = __fmaf_rn(__fmaf_rn(-den, y, 1.0f), y, y);
-    q = num * y;
-    q = __fmaf_rn(__fmaf_rn(-den, q, num), y, q);
-    ok = ok && (none || m2h >= 0x1p-100f) && den >= 0x1p-60f && den <= 0x1p60f && fabsf(num) <= 0x1p60f;
-    return q;
+    const float u = quotient(num, den, y);
+    range.nonzero(m1);
+    range.nonzero(m2);
+    range.nonzero(num);
+    range.lo = min(range.lo, __float_as_uint(den));
+    range.hi = max(max(range.hi, __float_as_uint(den)), __float_as_uint(m2));
+    range.small = range.small && fabsf(u) <= 0x1p60f;
+    return u;
 }
 
 // One plane's update with its moments already loaded (m1, m2 updated in place;
@@ -276,10 +297,11 @@ __device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, 
 // Written with the division and root alone, the pass was bound by their
 // instructions (176 an element, 79 % of the issue slots: zeros and small values
 // take the slow path of each), not by memory; a test per element around a shorter
-// form cost as much as it saved, so four elements share one. Adam alone on 1M
-// Gaussians 367 -> 266 us (1.66 GB of traffic: 6.2 TB/s, memory bound), on 200k
-// 91 -> 66; the fused step's SH half (1M, 8 views) 445 -> 284, geometry half 176 ->
-// 143.
+// form cost as much as it saved, so four elements share one, kept as integer minima
+// and maxima (15 us of the fused step's SH half less than comparisons). Adam alone on
+// 1M Gaussians 367 -> 270 us (1.66 GB of traffic: 6.1 TB/s, memory bound), on 200k
+// 91 -> 67; the fused step's SH half (1M, 8 views) 445 -> 282, geometry half 176 ->
+// 129. Where most moments have decayed to subnormals, 200k take 119 (150 before).
 __device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4& m1, float4& m2, const AdamArgs& a,
                                               const AdamStep& s) {
     const float* lr = a.lr + p * 4;
@@ -294,11 +316,11 @@ __device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4
         m1.w = a.b1 * m1.w + a.one_minus_b1 * g.w;
         m2.w = a.b2 * m2.w + a.one_minus_b2 * g.w * g.w;
     }
-    bool ok = true;
-    float4 u = make_float4(adam_divide_fast(m1.x, m2.x, lr[0], a, s, ok), adam_divide_fast(m1.y, m2.y, lr[1], a, s, ok),
-                           adam_divide_fast(m1.z, m2.z, lr[2], a, s, ok), 0.0f);
-    if (w) u.w = adam_divide_fast(m1.w, m2.w, lr[3], a, s, ok);
-    if (!ok) {
+    AdamRange range;
+    float4 u = make_float4(adam_divide_fast(m1.x, m2.x, lr[0], a, s, range), adam_divide_fast(m1.y, m2.y, lr[1], a, s, range),
+                           adam_divide_fast(m1.z, m2.z, lr[2], a, s, range), 0.0f);
+    if (w) u.w = adam_divide_fast(m1.w, m2.w, lr[3], a, s, range);
+    if (!range.all()) {
         u.x = adam_divide(m1.x, m2.x, lr[0], a, s);
         u.y = adam_divide(m1.y, m2.y, lr[1], a, s);
         u.z = adam_divide(m1.z, m2.z, lr[2], a, s);
