@@ -387,12 +387,12 @@ int rgs_get_memory(rgs_ctx* ctx, uint64_t* held_bytes, uint64_t* peak_bytes, int
 int rgs_trainer_evaluated_pairs(rgs_ctx* ctx, uint64_t* forward_pairs, uint64_t* backward_pairs);
 
 /* ---- tiling and its autotuner ---------------------------------------------
- * Tile shape, splats staged per batch and pixels per thread change only how
- * the blend kernels are laid out, never a result (every combination is
- * bit-identical), so they may change between training steps. */
+ * Tile shape and pixels per thread change only how the blend kernels are laid
+ * out, never an image (every combination is bit-identical), so they may change
+ * between training steps. batch is checked and reported, and changes nothing. */
 int rgs_get_options(rgs_ctx* ctx, rgs_options* out);
 /* Switches the blend layout (same value sets as rgs_create); the next batched
- * step recaptures its graph. */
+ * step recaptures its graph if the tile shape or the pixels per thread changed. */
 int rgs_set_tiling(rgs_ctx* ctx, int tile_w, int tile_h, int batch, int pixels_per_thread);
 
 /* One autotuner measurement: device milliseconds per render + backward of the
@@ -402,10 +402,11 @@ typedef struct rgs_tune_entry {
     float ms;
 } rgs_tune_entry;
 #define RGS_TUNE_CANDIDATES 18 /* {16x16, 8x32, 32x8} x {128, 256, 512} x {1, 2} */
-/* Times every candidate layout on the trainer's current Gaussians and the
- * given views (render, loss and backward; parameters and Adam state are not
- * touched), keeps the fastest and returns it in *chosen. results may be NULL
- * or hold RGS_TUNE_CANDIDATES entries. */
+/* Times every tile shape with either number of pixels per thread on the trainer's
+ * current Gaussians and the given views (render, loss and backward; parameters
+ * and Adam state are not touched), keeps the fastest and returns it in *chosen
+ * (with batch 128). results may be NULL or hold RGS_TUNE_CANDIDATES entries; the
+ * three batch rows of a layout share its time. */
 int rgs_trainer_autotune(rgs_ctx* ctx, const uint32_t* views, size_t nviews, const float bg[3],
                          const rgs_loss_config* loss_cfg, int reps, rgs_tune_entry* results,
                          rgs_options* chosen);

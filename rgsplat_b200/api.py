@@ -612,9 +612,10 @@ class Trainer:
 
     def autotune(self, views: Sequence[int], bg=(0.0, 0.0, 0.0), loss_cfg: LossConfig | None = None,
                  reps: int = 3) -> tuple[dict, list[dict]]:
-        """Times every blend layout (tile 16x16 / 8x32 / 32x8 x batch 128 / 256 /
-        512 x 1 or 2 pixels per thread) on a batched render + backward of
-        ``views`` and keeps the fastest. Returns (chosen, all measurements).
+        """Times every blend layout (tile 16x16 / 8x32 / 32x8 x 1 or 2 pixels per
+        thread) on a batched render + backward of ``views`` and keeps the fastest.
+        Returns (chosen, all measurements: the batch rows 128 / 256 / 512 of a
+        layout share its time).
         Parameters and the Adam state are not modified."""
         v = np.ascontiguousarray(views, dtype=np.uint32)
         lc = (loss_cfg or LossConfig()).to_c()
