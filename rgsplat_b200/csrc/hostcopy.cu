@@ -14,12 +14,15 @@
 //
 // The slabs belong to the process, not to a context: one block of HC_SLABS, handed
 // out under a mutex and given back when the last context is destroyed. It is
-// huge-page memory registered as a whole (16 MiB: 2 to 4 ms; sixteen cudaHostAlloc of
-// 1 MiB took 10 to 22; slabs of 512 KiB wrote 236 MB in 8.0 ms instead of 5.9). So
-// that a program that makes a context, copies a little and destroys it does not
-// pay even that, the block is made only once HC_FIRST bytes have gone by in large
-// copies. A copy that finds no slab free, or that is on a stream its threads cannot
-// name (cudaStreamPerThread), is the plain copy.
+// huge-page memory registered as a whole (16 MiB: 2.1 ms, and 0.7 to give back;
+// sixteen cudaHostAlloc of 1 MiB took 10 to 22; slabs of 512 KiB wrote 236 MB in 8.0
+// ms instead of 5.9). The block is made once HC_FIRST bytes have gone by in large
+// copies, when the plain copies have lost about what it costs: 32 MiB read in arrays
+// of 9 to 24 MB lose 1 to 1.5 ms, in one array of 47 MB 7 ms, written 0.4 to 1. A
+// program that copies less and ends never pays; one that goes on pays 2.8 ms for what
+// each such call then saves (a drop-in call of 50k Gaussians, 24 MB, 3.7 -> 2.7).
+// A copy that finds no slab free, or that is on a stream its threads cannot name
+// (cudaStreamPerThread), is the plain copy.
 #include <sys/mman.h>
 
 #include <algorithm>

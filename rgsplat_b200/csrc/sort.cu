@@ -501,8 +501,9 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n_host, const uint
     }
     int cur = 0;
     int shift = 0;
-    // 8-bit digits; a final pass over fewer significant bits still reads 8
-    // (the bits above `bits` are zero in every key, so they do not reorder).
+    // 8-bit digits; a final pass over fewer significant bits still reads 8 (the
+    // bits from `bits` to the digit's end are zero in every key, so they do not
+    // reorder; what is above, the tile masks of packed entries, no pass reads)
     while (shift < bits) {
         uint32_t* hist = sc.hist.as<uint32_t>();
         uint32_t* dtot = hist + (size_t)grid * 256;

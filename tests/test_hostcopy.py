@@ -18,7 +18,8 @@ MIB = 1 << 20
 def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("hostcopy") / "hostcopy.so")
     cuda = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
-    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-I" + cuda, "-I" + build.CSRC,
+    # -Bsymbolic: the stand-in's functions, also where the process has loaded the real ones
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-I" + cuda, "-I" + build.CSRC,
                     "-I" + build.INCLUDE, "-x", "c++", os.path.join(build.CSRC, "hostcopy.cu"),
                     os.path.join(HERE, "hostcopy_fake.cpp"), "-o", out], check=True)
     lib = ctypes.CDLL(out)
