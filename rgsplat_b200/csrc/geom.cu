@@ -250,7 +250,7 @@ __device__ __forceinline__ float adam_divide(float m1, float m2, float lr, const
 // Res. Dev. 34(1), 1990): the product, corrected by the exact remainder. The product
 // is off by less than half an ulp for y and half for itself, so near a tie it is one
 // of the tie's two neighbours and the correction rounds as the quotient does. a is 0
-// (and the quotient the same zero) or at least 2^-100, so that the remainder is exact.
+// (and the quotient the same zero) or at least 2^-102, so that the remainder is exact.
 __device__ __forceinline__ float quotient(float a, float b, float y) {
     const float q = a * y;
     return __fmaf_rn(-__fmaf_rn(q, b, -a), y, q);
@@ -258,32 +258,34 @@ __device__ __forceinline__ float quotient(float a, float b, float y) {
 
 // Whether values met so far are in the range of adam_divide_fast.
 struct AdamRange {
-    uint32_t least = 0xffffffffu;       // of 2 bits(x) - 1, x zero or at least 2^-100
+    uint32_t least = 0xffffffffu;       // of 2 bits(x) - 1, x zero or at least 2^-102
     uint32_t lo = 0xffffffffu, hi = 0;  // of the denominators' bits (hi: and of m2's, below 0 too large)
     bool small = true;                  // every |update| <= 2^60
     __device__ __forceinline__ void nonzero(float x) { least = min(least, 2u * __float_as_uint(x) - 1u); }
     __device__ __forceinline__ bool all() const {
-        return small && least >= 2u * (27u << 23) - 1u && lo >= 67u << 23 && hi <= 147u << 23;  // 2^-100, 2^-60, 2^20
+        return small && least >= 2u * (25u << 23) - 1u && lo >= 67u << 23 && hi <= 147u << 23;  // 2^-102, 2^-60, 2^20
     }
 };
 
 // The same update without a branch and with the same roundings, for values in a
 // range that `range` reports. The denominator's reciprocal and the root are one
 // hardware approximation and one such correction each; both were compared with the
-// rounded values over every mantissa (the root over every float of [2^-100, 2^40]),
+// rounded values over every mantissa (the root over every float of [2^-102, 2^64]),
 // and the quotients over 2^33 pairs, 9 10^7 of the nearest to a tie among them: none
-// differs. 0 <= m2, and m2 = 0 has root 0.
+// differs. 0 <= m2, and m2 = 0 has root 0; m2, a gradient's square, is scaled by 2^24
+// and its root back, both exactly, so that it may be any normal number up to 2^20.
 __device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, const AdamArgs& a, const AdamStep& s, AdamRange& range) {
-    const float m1h = quotient(m1, s.bc1, s.r1), m2h = quotient(m2, s.bc2, s.r2);
+    const float m2s = m2 * 0x1p24f;
+    const float m1h = quotient(m1, s.bc1, s.r1), m2h = quotient(m2s, s.bc2, s.r2);
     float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(m2h, 0x1p-100f)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(m2h, 0x1p-102f)));
     float q = m2h * y;
-    const float num = lr * m1h, den = __fmaf_rn(__fmaf_rn(-q, q, m2h), 0.5f * y, q) + a.eps;
+    const float num = lr * m1h, den = __fmaf_rn(__fmaf_rn(__fmaf_rn(-q, q, m2h), 0.5f * y, q), 0x1p-12f, a.eps);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den));
     y = __fmaf_rn(__fmaf_rn(-den, y, 1.0f), y, y);
     const float u = quotient(num, den, y);
     range.nonzero(m1);
-    range.nonzero(m2);
+    range.nonzero(m2s);
     range.nonzero(num);
     range.lo = min(range.lo, __float_as_uint(den));
     range.hi = max(max(range.hi, __float_as_uint(den)), __float_as_uint(m2));
@@ -298,10 +300,10 @@ __device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, 
 // instructions (176 an element, 79 % of the issue slots: zeros and small values
 // take the slow path of each), not by memory; a test per element around a shorter
 // form cost as much as it saved, so four elements share one, kept as integer minima
-// and maxima (15 us of the fused step's SH half less than comparisons). Adam alone on
-// 1M Gaussians 367 -> 270 us (1.66 GB of traffic: 6.1 TB/s, memory bound), on 200k
-// 91 -> 67; the fused step's SH half (1M, 8 views) 445 -> 282, geometry half 176 ->
-// 129. Where most moments have decayed to subnormals, 200k take 119 (150 before).
+// and maxima (24 us of the fused step's SH half less than comparisons). Adam alone on
+// 1M Gaussians 367 -> 265 us (1.66 GB of traffic: 6.3 TB/s, memory bound), on 200k
+// 91 -> 66; the fused step's SH half (1M, 8 views) 445 -> 271, geometry half 176 ->
+// 128. Where most moments have decayed to subnormals, 200k take 122 (150 before).
 __device__ __forceinline__ float4 adam_update(int p, float4 pv, float4 g, float4& m1, float4& m2, const AdamArgs& a,
                                               const AdamStep& s) {
     const float* lr = a.lr + p * 4;
