@@ -108,7 +108,7 @@ __device__ __forceinline__ bool not_sane(const float4& Q, const float4& K) {
 // or colour is not finite goes through a scalar loop, so 0 * NaN reaches no
 // pixel that does not take it.)
 //
-// What bounds it: the FMA pipe (72 % of cycles; two thirds of its work is the
+// What bounds it: the FMA pipe (73 % of cycles; two thirds of its work is the
 // reference's exact exponential, 18 packed instructions per pixel pair), so what
 // matters is not to evaluate pairs that cannot contribute. Each warp walks the
 // bit mask of the staged splats that can reach its own strip of rows (about half
@@ -356,7 +356,7 @@ __device__ __noinline__ float2 bwd_exact_pixel(float dx, float dy, float4 q, flo
 // rebuilt as T * 1/(1 - alpha) with the hardware reciprocal (within 2 ulp; the
 // reference divides, backward.rs:452).
 //
-// What bounds it: instruction issue (78 % of cycles; FMA pipe 54 %, ALU 40 %),
+// What bounds it: instruction issue (78 % of cycles; FMA pipe 59 %, ALU 39 %),
 // so the loop is built around the fewest instructions per (warp, splat). It
 // replaces a loop that tested both thresholds on each pixel's alpha and reduced
 // nine sums over the warp for every splat: 3.29 -> 1.52 ms on 1M Gaussians x 8

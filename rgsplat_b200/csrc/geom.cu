@@ -300,7 +300,7 @@ __device__ __forceinline__ float adam_divide_fast(float m1, float m2, float lr, 
 // instructions (176 an element, 79 % of the issue slots: zeros and small values
 // take the slow path of each), not by memory; a test per element around a shorter
 // form cost as much as it saved, so four elements share one, kept as integer minima
-// and maxima (24 us of the fused step's SH half less than comparisons). Adam alone on
+// and maxima (35 us of the fused step's SH half less than comparisons). Adam alone on
 // 1M Gaussians 367 -> 265 us (1.66 GB of traffic: 6.3 TB/s, memory bound), on 200k
 // 91 -> 66; the fused step's SH half (1M, 8 views) 445 -> 271, geometry half 176 ->
 // 128. Where most moments have decayed to subnormals, 200k take 122 (150 before).

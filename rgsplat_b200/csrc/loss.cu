@@ -65,8 +65,10 @@ __device__ __forceinline__ float ssim_maps(float mx, float my, float exx, float 
 // as (P, Q), (R, Q mu_y), R mu_x. Pass outputs live in shared memory as float2
 // planes of those pairs (plus one float plane).
 //
-// What bounds it: FMA issue (339 fused multiply-adds per pixel and channel with
-// the halos) and the latency around the four barriers per channel. Ten warps
+// What bounds it: the shared-memory pipe (60 % of cycles, a quarter of its
+// wavefronts bank conflicts) and the latency around the four barriers per channel,
+// with 18 warps an SM; the FMA pipe (339 fused multiply-adds per pixel and channel
+// with the halos) is 47 % busy. Ten warps
 // share a 32x32 tile: with runs of 7, 6, 8 and 4 outputs the four passes have
 // 312, 294, 168 and 256 work items for 320 threads (256 threads leave the first
 // pass a second round that is three quarters empty). The maps reuse the input's
