@@ -71,14 +71,9 @@ __device__ __forceinline__ void cta_tile_box(int tx, int ty, int tw, int th, int
 // for xl (the roots are formed with 1/a, within an ulp of the quotient). The
 // span is computed with T enlarged by 2 % and widened by half a pixel, so it
 // contains every tile the per-tile test keeps with a margin far above float
-// rounding (and above that of the approximate square roots and quotients used
-// here); the blend still applies its own tests.
-__device__ __forceinline__ float sqrt_approx(float x) {
-    float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
+// rounding; the blend still applies its own tests. (Approximate square roots and
+// quotients would be covered by that margin too, and 2 % of a 3M-Gaussian step
+// faster, but they move a pair in 10^7 in or out of the lists and the pair count.)
 struct SpanSetup {
     float sx, sy, a, b, c, T, xr, yr, ia;  // ia = 1 / a
     bool testable;
@@ -90,9 +85,9 @@ __device__ __forceinline__ SpanSetup span_setup(float sx, float sy, float a, flo
     u.testable = a > 0.0f && c > 0.0f && (a * c - b * b) >= 0.01f * (a * c);
     u.T = -2.0f * thr / 0.999f * 1.02f;
     const float det = a * c - b * b;
-    u.xr = u.testable ? sqrt_approx(__fdividef(u.T * c, det)) : 0.0f;
-    u.yr = u.testable ? __fdividef(-b, c) * u.xr : 0.0f;
-    u.ia = u.testable ? __fdividef(1.0f, a) : 0.0f;
+    u.xr = u.testable ? sqrtf(u.T * c / det) : 0.0f;
+    u.yr = u.testable ? -b / c * u.xr : 0.0f;
+    u.ia = u.testable ? 1.0f / a : 0.0f;
     return u;
 }
 
@@ -114,7 +109,7 @@ __device__ __forceinline__ void kept_cols(const SpanSetup& u, int ty, int tw, in
             c1 = c0;
             return;
         }
-        xr = (-u.b * er + sqrt_approx(disc)) * u.ia;
+        xr = (-u.b * er + sqrtf(disc)) * u.ia;
     }
     const float el = fminf(fmaxf(-u.yr, ly), hy);
     if (el == -u.yr) {
@@ -125,7 +120,7 @@ __device__ __forceinline__ void kept_cols(const SpanSetup& u, int ty, int tw, in
             c1 = c0;
             return;
         }
-        xl = (-u.b * el - sqrt_approx(disc)) * u.ia;
+        xl = (-u.b * el - sqrtf(disc)) * u.ia;
     }
     // pixel-space interval, widened by half a pixel; a tile's pixel centres
     // span [tx * tw + 0.5, tx * tw + tw - 0.5]
