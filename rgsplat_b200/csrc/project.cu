@@ -168,7 +168,7 @@ __device__ __forceinline__ uint32_t rect_supertiles(int cx0, int cx1, int cy0, i
 // Kept spans of rectangles over SPAN_ROWS rows or 15 columns are found by the
 // whole warp, one such slot after another and one lane per tile row: a thread
 // walking its own rows kept the warp for the tallest of its rectangles (3M
-// anisotropic Gaussians, 8 views of 1920x1080, 2.6 -> 2.1 ms a
+// anisotropic Gaussians, 8 views of 1920x1080, 2.6 -> 2.2 ms a
 // launch).
 __global__ void __launch_bounds__(256, 5) k_project(const float4* __restrict__ params, int n, int cap,
                                                  const DevCam* __restrict__ cams, int nviews, int tile_w,
